@@ -220,7 +220,7 @@ struct gcf_ctx {
     DBuf<__nv_bfloat16> rsg_bf;   // scratch of the tensor-core rescale (gcf_rsgemm.cu)
     DBuf<float> rsg_f;
     DBuf<int> rsg_err;            // its products' bounded-wait flag, checked when results are read
-    DBuf<double> acc, hsum, moments, moments2;
+    DBuf<double> acc, hsum, moments, moments2, tile_sums;
     DBuf<float> lpfull;
     DBuf<float2> lpcmp;
     DBuf<float> raw, ctf0, ctf, radial, band_spec, cc_res, full;
@@ -699,15 +699,16 @@ gcf_status spectrum_cufft(gcf_ctx* ctx, const MicImage& m, float* raw_out)
     const int kBatch = 256;
     int batch = std::min(nt, kBatch);
     CK(ctx->tiles.ensure((size_t)batch * T * T));
+    CK(ctx->tile_sums.ensure((size_t)batch * kMeanSlices));
     CK(ctx->cmp.ensure((size_t)batch * cx * T));
     CK(ctx->acc.ensure((size_t)cx * T));
     CK(cudaMemsetAsync(ctx->acc.p, 0, (size_t)cx * T * sizeof(double), ctx->st));
     for (int t0 = 0; t0 < nt; t0 += batch) {
         int nb = std::min(batch, nt - t0);
-        launch_extract_tiles(m.img, m.w, m.h, m.pitch, T, L.ntx, L.offx, L.offy, L.stride, t0, nb,
-                             ctx->taper.p, ctx->tiles.p, ctx->st);
+        launch_extract_tiles(m.img, m.pitch, T, L.ntx, L.offx, L.offy, L.stride, t0, nb, ctx->taper.p,
+                             ctx->tile_sums.p, ctx->tiles.p, ctx->st);
         CKL();
-        ctx->launches += 1;
+        ctx->launches += 2;
         cufftHandle plan;
         CKS(get_plan(ctx, 0, T, nb, &plan));
         if (cufftExecR2C(plan, ctx->tiles.p, (cufftComplex*)ctx->cmp.p) != CUFFT_SUCCESS)
@@ -1934,6 +1935,7 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->rsg_f.release();
     ctx->rsg_err.release();
     ctx->acc.release();
+    ctx->tile_sums.release();
     ctx->hsum.release();
     ctx->lpfull.release();
     ctx->lpcmp.release();

@@ -184,9 +184,11 @@ struct EvalArgs {
 // ---------------------------------------------------------------------------
 
 // gcf_spectrum.cu
-void launch_extract_tiles(const float* img, int w, int h, int pitch, int tile, int ntx,
-                          int offx, int offy, int stride, int first_tile, int ntiles,
-                          const float* taper, float* out, cudaStream_t st);
+constexpr int kMeanSlices = 16;   // row slices of a tile's FP64 sum
+// sums: kMeanSlices doubles per tile of scratch
+void launch_extract_tiles(const float* img, int pitch, int tile, int ntx, int offx, int offy, int stride,
+                          int first_tile, int ntiles, const float* taper, double* sums, float* out,
+                          cudaStream_t st);
 void launch_amp_accumulate(const float2* cmp, int tile, int ntiles, double* acc, cudaStream_t st);
 void launch_finalize_raw(const double* acc, int n, double inv, float* raw, cudaStream_t st);
 void launch_fourier_crop(const float2* in, int cx_in, int cy_in, float2* out, int cx_out,
