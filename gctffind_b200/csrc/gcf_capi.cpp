@@ -231,6 +231,8 @@ struct gcf_ctx {
     DBuf<float2> cval;
     DBuf<double2> part;
     DBuf<int> arrive;
+    DBuf<Best1D> best_1d;
+    DBuf<First1D> first_1d;
     DBuf<gcf_result> d_res;
     DBuf<PixOptics> d_optics;
 
@@ -1036,7 +1038,7 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     std::vector<SearchJob> jh(nj);
     std::vector<int> soff(nj);
     int tot = 0, max_band = 0;
-    bool any_full = false, any_grid = false, any_phase = false, any_1d = false;
+    bool any_full = false, any_grid = false, any_phase = false, any_1d = false, any_phase_1d = false;
     for (int j = 0; j < nj; ++j) {
         const JobSpec& s = specs[j];
         SearchJob& J = jh[j];
@@ -1053,6 +1055,7 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
         J.r1d_df = s.r1d_df;
         J.r1d_range = s.r1d_range;
         J.step = STEP_CC0;
+        if (J.phase_range_in > 0) any_phase_1d = true;
         if (s.mode >= 2) {
             any_1d = true;
         } else if (s.mode == 1) {
@@ -1083,6 +1086,10 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     CK(ctx->cc_res.ensure((size_t)nj * cx));
     CK(ctx->d_res.ensure(nj));
     CK(ctx->arrive.ensure(nj));
+    if (ctx->n_sms == 0) CK(cudaDeviceGetAttribute(&ctx->n_sms, cudaDevAttrMultiProcessorCount, ctx->dev));
+    const int ctas_1d = search1d_ctas(nj, any_phase_1d, ctx->n_sms);
+    CK(ctx->best_1d.ensure((size_t)nj * ctas_1d));
+    CK(ctx->first_1d.ensure(nj));
     CK(cudaMemsetAsync(ctx->arrive.p, 0, nj * sizeof(int), ctx->st));
     CK(h2d(ctx, ctx->jobs.p, jh.data(), nj * sizeof(SearchJob), ctx->st));
     CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int), ctx->st));
@@ -1104,9 +1111,10 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     a.njobs = nj;
     CK(record_timing(ctx->ev[5], ctx->st));
     if (any_full || any_1d) {
-        launch_search1d(ctx->jobs.p, nj, ctx->radial.p, cx, ctx->cand.p, ctx->cval.p, ctx->st);
+        launch_search1d(ctx->jobs.p, nj, ctas_1d, ctx->radial.p, cx, ctx->cand.p, ctx->cval.p, ctx->best_1d.p,
+                        ctx->first_1d.p, ctx->arrive.p, ctx->st);
         CKL();
-        ctx->launches += 1;
+        ctx->launches += 2;
     }
     launch_init_jobs(a, ctx->st);   // Refine jobs: pending step CC0
     CKL();
@@ -1121,7 +1129,6 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     // it is given, reusing its pixels, so with many jobs fewer y-blocks
     // (enough for about two waves of 3 CTAs per SM) do the same work without
     // the blocks that find no candidates and exit.
-    if (ctx->n_sms == 0) CK(cudaDeviceGetAttribute(&ctx->n_sms, cudaDevAttrMultiProcessorCount, ctx->dev));
     const long long per_y = (long long)nj * max_chunks;
     const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (2LL * 3 * ctx->n_sms + per_y - 1) / per_y));
     for (int k = 0; k < pairs; ++k) {
@@ -1957,6 +1964,9 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->cand.release();
     ctx->cval.release();
     ctx->part.release();
+    ctx->arrive.release();
+    ctx->best_1d.release();
+    ctx->first_1d.release();
     ctx->d_res.release();
     ctx->d_optics.release();
     ctx->d_counts.release();

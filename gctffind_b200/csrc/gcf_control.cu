@@ -30,6 +30,7 @@ namespace {
 constexpr float kD2R2D = 0.01745329f;   // FindCTF/CFindDefocus2D.cpp:11
 constexpr float kD2R1D = 0.0174533f;    // FindCTF/CFindDefocus1D.cpp:11
 constexpr double kPi = 3.14159265358979323846;
+constexpr int k1DThreads = 256;
 
 struct Cand {
     float ast, ang, phase, dfmean;
@@ -718,15 +719,25 @@ struct Bins1D {
     float a[kMax1DBins], d[kMax1DBins], env[kMax1DBins], s[kMax1DBins];
 };
 
-struct Brute {
-    float df, ph, cc;
-    int n;   // grid points evaluated
+// CFindDefocus1D::mBrutalForceSearch's grid (FindCTF/CFindDefocus1D.cpp:76-119):
+// ndf defocus values x nps extra phases, defocus innermost.
+struct Grid1D {
+    int ndf, nps;
+    float df0, dfs, ph0, pss;
+    __device__ int points() const { return ndf * nps; }
+    __device__ float df(int i) const { return df0 + (i % ndf) * dfs; }
+    __device__ float phase(int i) const
+    {
+        float ph = ph0 + (i / ndf) * pss;
+        if (ph < 0) ph = 0.0f;
+        else if (ph > 150.0f) ph = 150.0f;
+        return ph;
+    }
 };
 
-__device__ Brute brute_1d(const Bins1D& B, int lo_bin, int hi_bin, double ss, const PixOptics& o,
-                          const float dfr[2], const float phr[2], ArgMax* shm)
+__device__ Grid1D grid_1d(const float dfr[2], const float phr[2])
 {
-    // CFindDefocus1D::mBrutalForceSearch (FindCTF/CFindDefocus1D.cpp:76-119)
+    Grid1D g;
     int ndf = 501;
     float dfrange = dfr[1] - dfr[0];
     float dfs = dfrange / (ndf - 1);
@@ -737,17 +748,51 @@ __device__ Brute brute_1d(const Bins1D& B, int lo_bin, int hi_bin, double ss, co
     float pss = psr / (nps - 1);
     if (pss == 0) nps = 1;
     else nps = (int)(psr / pss) / 2 * 2 + 1;
-    int npts = ndf * nps;
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    g.ndf = ndf;
+    g.nps = nps;
+    g.df0 = dfr[0];
+    g.dfs = dfs;
+    g.ph0 = phr[0];
+    g.pss = pss;
+    return g;
+}
+
+// Grid of pass 1 (CFindCtf1D::mFindDefocus, FindCTF/CFindCtf1D.cpp:73-90).
+__device__ Grid1D first_grid_1d(const SearchJob& J)
+{
+    const float px2 = J.o.px * J.o.px;
+    float dfr[2] = {3000.0f * px2, 30000.0f * px2};
+    float phr[2];
+    phr[0] = fmaxf(J.ext_phase_in - J.phase_range_in / 2, 0.0f);
+    phr[1] = fminf(phr[0] + J.phase_range_in, 150.0f);
+    return grid_1d(dfr, phr);
+}
+
+// Grid of pass 2 (CFindCtf1D::mRefineDefocus, FindCTF/CFindCtf1D.cpp:92-111)
+// around pass 1's best defocus and phase.
+__device__ Grid1D refine_grid_1d(const SearchJob& J, float df, float ph, float range)
+{
+    float mindf = 3000.0f * J.o.px * J.o.px;
+    float dfr[2], phr[2];
+    dfr[0] = fmaxf(df - range / 2, mindf);
+    dfr[1] = dfr[0] + range;
+    float pr = 0.2f * J.phase_range_in;
+    phr[0] = fmaxf(ph - pr / 2, 0.0f);
+    phr[1] = fminf(0.0f + pr, 150.0f);   // the reference reads the zero-initialised bound
+    return grid_1d(dfr, phr);
+}
+
+// The best of the grid points i = w, w + nw, ... of this warp (w: the
+// warp's index among the job's nw warps, over all of its CTAs), in index
+// order.
+__device__ ArgMax brute_1d(const Bins1D& B, int lo_bin, int hi_bin, double ss, const PixOptics& o,
+                           const Grid1D& g, int w, int nw)
+{
+    const int lane = threadIdx.x & 31, npts = g.points();
     ArgMax m{(float)-1e20, -1};
-    for (int i = warp; i < npts; i += nw) {
-        int f = i % ndf, p = i / ndf;
-        float df = dfr[0] + f * dfs;
-        float ph = phr[0] + p * pss;
-        if (ph < 0) ph = 0.0f;
-        else if (ph > 150.0f) ph = 150.0f;
-        float pdf = df / o.px;
-        float add = o.amp_phase + ph * kD2R1D;
+    for (int i = w; i < npts; i += nw) {
+        float pdf = g.df(i) / o.px;
+        float add = o.amp_phase + g.phase(i) * kD2R1D;
         float tw = (float)((double)add / kPi);
         float cs = 0.f, cc = 0.f;
         for (int x = lo_bin + lane; x < hi_bin; x += 32) {
@@ -766,33 +811,38 @@ __device__ Brute brute_1d(const Bins1D& B, int lo_bin, int hi_bin, double ss, co
         float v = (dcc > 0 && ss > 0) ? (float)(dcs / sqrt(dcc * ss)) : 0.0f;
         if (v > m.v) m = ArgMax{v, i};
     }
-    __syncthreads();
-    m = block_argmax(m, shm);
-    Brute r{0.0f, 0.0f, (float)-1e20, npts};
-    if (m.i >= 0) {
-        int f = m.i % ndf, p = m.i / ndf;
-        float ph = phr[0] + p * pss;
-        if (ph < 0) ph = 0.0f;
-        else if (ph > 150.0f) ph = 150.0f;
-        r.df = dfr[0] + f * dfs;
-        r.ph = ph;
-        r.cc = m.v;
-    }
-    return r;
+    return m;
 }
 
-__global__ void k_search1d(SearchJob* __restrict__ jobs, const float* __restrict__ radial, int cx,
-                           float4* __restrict__ cand, float2* __restrict__ cval)
+// One pass of the 1D search (grid: CTAs per job x jobs): every CTA of a job
+// takes its share of the pass's grid points, and the job's last CTA to
+// finish (an arrival counter, no waiting) picks the first strict maximum in
+// index order.  pass 1 leaves it in first[j]; pass 2 sets up the 2D search.
+//
+// Bound: latency and the sine unit.  One CTA per job ran the 2 x 501 points
+// of one job in 117 us on one SM, and the 2 x 18537 points of an extra-phase
+// search in 3788 us; spread over up to 64 CTAs (about four points per warp)
+// the two passes take 21 and 70 us.
+__global__ void __launch_bounds__(k1DThreads)
+k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ radial, int cx,
+           float4* __restrict__ cand, float2* __restrict__ cval, Best1D* __restrict__ best,
+           First1D* __restrict__ first, int* __restrict__ arrive)
 {
     extern __shared__ unsigned char smem_raw[];
     Bins1D& B = *reinterpret_cast<Bins1D*>(smem_raw);
     __shared__ ArgMax shm[32];
     __shared__ double s_ss;
     __shared__ SearchJob sJ;
-    const int j = blockIdx.x;
-    if (threadIdx.x == 0) sJ = jobs[j];
+    __shared__ int s_last, s_lo, s_hi;
+    const int j = blockIdx.y;
+    if (threadIdx.x == 0) {
+        sJ = jobs[j];
+        s_lo = cx;
+        s_hi = 0;
+    }
     __syncthreads();
     if (sJ.mode == 1 || sJ.mode == 4) return;   // Refine and the contraction search have no 1D stage here
+    if (pass == 1 && sJ.mode == 3) return;      // Refine1D: the refinement pass only
     const PixOptics o = sJ.o;
     const float* rad = radial + (size_t)sJ.mic * cx;
     // CFindDefocus1D::mCorrelate band (FindCTF/CFindDefocus1D.cpp:128-137)
@@ -800,14 +850,11 @@ __global__ void k_search1d(SearchJob* __restrict__ jobs, const float* __restrict
     if (r1 < 3.5f) r1 = 3.5f;
     float res1 = ((cx - 1) * 2) * o.px;
     float flo = res1 / r0, fhi = res1 / r1;
-    int lo_bin = cx, hi_bin = 0;
-    for (int x = 0; x < cx; ++x) {
-        if ((float)x >= flo && (float)x < fhi) {
-            if (x < lo_bin) lo_bin = x;
-            hi_bin = x + 1;
-        }
-    }
     for (int x = threadIdx.x; x < cx; x += blockDim.x) {
+        if ((float)x >= flo && (float)x < fhi) {
+            atomicMin(&s_lo, x);
+            atomicMax(&s_hi, x + 1);
+        }
         double s = (x * 0.5) / (cx - 1.0);
         double s2 = s * s;
         double f = x / (cx - 1.0);
@@ -817,6 +864,7 @@ __global__ void k_search1d(SearchJob* __restrict__ jobs, const float* __restrict
         B.s[x] = rad[x];
     }
     __syncthreads();
+    const int lo_bin = s_lo, hi_bin = s_hi;
     if (threadIdx.x < 32) {
         double ss = 0.0;
         for (int x = lo_bin + (int)threadIdx.x; x < hi_bin; x += 32) ss += (double)B.s[x] * B.s[x];
@@ -824,73 +872,81 @@ __global__ void k_search1d(SearchJob* __restrict__ jobs, const float* __restrict
         if (threadIdx.x == 0) s_ss = ss;
     }
     __syncthreads();
-    const double ss = s_ss;
-    // CFindCtf1D::mFindDefocus (FindCTF/CFindCtf1D.cpp:73-90)
-    float ext = sJ.ext_phase_in, prange = sJ.phase_range_in;
-    float px2 = o.px * o.px;
-    Brute b1;
-    float range;
-    if (sJ.mode == 3) {
-        // CFindCtf1D::Refine1D (FindCTF/CFindCtf1D.cpp:58-67): refine pass only,
-        // around the given defocus and the current extra phase
-        b1 = Brute{sJ.r1d_df, ext, 0.0f, 0};
-        range = sJ.r1d_range;
+    Grid1D g;
+    First1D f1{sJ.r1d_df, sJ.ext_phase_in, 0};   // Refine1D: around the given defocus and the current phase
+    if (pass == 1) {
+        g = first_grid_1d(sJ);
     } else {
-        float dfr[2] = {3000.0f * px2, 30000.0f * px2};
-        float phr[2];
-        phr[0] = fmaxf(ext - prange / 2, 0.0f);
-        phr[1] = fminf(phr[0] + prange, 150.0f);
-        b1 = brute_1d(B, lo_bin, hi_bin, ss, o, dfr, phr, shm);
-        range = fmaxf(0.3f * b1.df, 3000.0f);   // CFindCtf1D::Do1D (FindCTF/CFindCtf1D.cpp:49-56)
-    }
-    // CFindCtf1D::mRefineDefocus (FindCTF/CFindCtf1D.cpp:92-111)
-    float mindf = 3000.0f * o.px * o.px;
-    float dfr2[2];
-    dfr2[0] = fmaxf(b1.df - range / 2, mindf);
-    dfr2[1] = dfr2[0] + range;
-    float pr = 0.2f * prange;
-    float phr2[2];
-    phr2[0] = fmaxf(b1.ph - pr / 2, 0.0f);
-    phr2[1] = fminf(0.0f + pr, 150.0f);   // the reference reads the zero-initialised bound
-    Brute b2 = brute_1d(B, lo_bin, hi_bin, ss, o, dfr2, phr2, shm);
-    if (threadIdx.x == 0) {
-        sJ.n_cand1d += b1.n + b2.n;
-        sJ.n_pairs1d += (b1.n + b2.n) * max(hi_bin - lo_bin, 0);
-    }
-    if (sJ.mode >= 2) {   // Do1D / Refine1D alone: no 2D search follows
-        if (threadIdx.x == 0) {
-            sJ.df_1d = b2.df;
-            sJ.phase_1d = b2.ph;
-            sJ.score_1d = b2.cc;
-            sJ.step = STEP_DONE;
-            sJ.ncand = 0;
-            jobs[j] = sJ;
+        float range = sJ.r1d_range;
+        if (sJ.mode != 3) {
+            f1 = first[j];
+            range = fmaxf(0.3f * f1.df, 3000.0f);   // CFindCtf1D::Do1D (FindCTF/CFindCtf1D.cpp:49-56)
         }
+        g = refine_grid_1d(sJ, f1.df, f1.ph, range);
+    }
+    const int nw = (blockDim.x >> 5) * gridDim.x;
+    ArgMax m = brute_1d(B, lo_bin, hi_bin, s_ss, o, g, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw);
+    __syncthreads();
+    m = block_argmax(m, shm);
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) {
+            best[(size_t)j * gridDim.x + blockIdx.x] = Best1D{m.v, m.i};
+            __threadfence();
+            s_last = (atomicAdd(arrive + j, 1) == (int)gridDim.x - 1);
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (threadIdx.x == 0) arrive[j] = 0;
+        m = ArgMax{0.0f, -1};
+        for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+            const Best1D q = best[(size_t)j * gridDim.x + k];
+            m = better(m, ArgMax{q.v, q.i});
+        }
+        __syncthreads();
+        m = block_argmax(m, shm);
+    }
+    float b_df = 0.0f, b_ph = 0.0f, b_cc = (float)-1e20;
+    if (m.i >= 0) {
+        b_df = g.df(m.i);
+        b_ph = g.phase(m.i);
+        b_cc = m.v;
+    }
+    if (pass == 1) {
+        if (threadIdx.x == 0) first[j] = First1D{b_df, b_ph, g.points()};
         return;
     }
     float2* vj = cval + (size_t)j * kMaxCand;
     __shared__ int s_n;
     if (threadIdx.x == 0) {
-        sJ.df_1d = b2.df;
-        sJ.phase_1d = b2.ph;
-        sJ.score_1d = b2.cc;
-        // CFindCtf2D::Do2D + CFindDefocus2D::Setup3/DoIt (FindCTF/CFindCtf2D.cpp:44-53,
-        // FindCTF/CFindDefocus2D.cpp:98-124)
-        float mu = (b2.df + b2.df) * 0.5f;
-        sJ.df_mean = mu;
-        sJ.ast_ratio = 0.0f;
-        sJ.ast_angle = 0.0f;
-        sJ.phase_range[0] = b2.ph;
-        sJ.phase_range[1] = prange;
-        sJ.ext_phase = sJ.held_phase;   // replaced by phase_range[0] after the astigmatism grid
-        sJ.df_range[0] = mu * 0.9f;
-        sJ.df_range[1] = mu * 1.1f;
-        sJ.ast_range[0] = 0.0f;
-        sJ.ast_range[1] = 0.06f;
-        sJ.ang_range[0] = -90.0f;
-        sJ.ang_range[1] = 90.0f;
-        sJ.step = STEP_CC0;
-        s_n = advance(sJ, vj);
+        const int n1d = f1.n + g.points();
+        sJ.n_cand1d += n1d;
+        sJ.n_pairs1d += n1d * max(hi_bin - lo_bin, 0);
+        sJ.df_1d = b_df;
+        sJ.phase_1d = b_ph;
+        sJ.score_1d = b_cc;
+        if (sJ.mode >= 2) {   // Do1D / Refine1D alone: no 2D search follows
+            sJ.step = STEP_DONE;
+            s_n = 0;
+        } else {
+            // CFindCtf2D::Do2D + CFindDefocus2D::Setup3/DoIt (FindCTF/CFindCtf2D.cpp:44-53,
+            // FindCTF/CFindDefocus2D.cpp:98-124)
+            float mu = (b_df + b_df) * 0.5f;
+            sJ.df_mean = mu;
+            sJ.ast_ratio = 0.0f;
+            sJ.ast_angle = 0.0f;
+            sJ.phase_range[0] = b_ph;
+            sJ.phase_range[1] = sJ.phase_range_in;
+            sJ.ext_phase = sJ.held_phase;   // replaced by phase_range[0] after the astigmatism grid
+            sJ.df_range[0] = mu * 0.9f;
+            sJ.df_range[1] = mu * 1.1f;
+            sJ.ast_range[0] = 0.0f;
+            sJ.ast_range[1] = 0.06f;
+            sJ.ang_range[0] = -90.0f;
+            sJ.ang_range[1] = 90.0f;
+            sJ.step = STEP_CC0;
+            s_n = advance(sJ, vj);
+        }
         sJ.ncand = s_n;
         jobs[j] = sJ;
     }
@@ -1194,12 +1250,23 @@ void launch_init_jobs(const EvalArgs& a, cudaStream_t st)
     k_init_jobs<<<a.njobs, 256, 0, st>>>(a.jobs, a.cand, a.cval);
 }
 
-void launch_search1d(SearchJob* jobs, int njobs, const float* radial, int cx, float4* cand,
-                     float2* cval, cudaStream_t st)
+int search1d_ctas(int njobs, bool phase, int sms)
+{
+    // about four grid points per warp (501 defocus values, 37 times as many
+    // with an extra-phase range), and no more CTAs than fill the chip four
+    // times over
+    const int want = phase ? 64 : 16;
+    return std::max(1, std::min(want, 4 * sms / std::max(njobs, 1)));
+}
+
+void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, float4* cand,
+                     float2* cval, Best1D* best, First1D* first, int* arrive, cudaStream_t st)
 {
     if (njobs <= 0) return;
     size_t sm = sizeof(Bins1D);   // 16.4 KB, below the default dynamic limit
-    k_search1d<<<njobs, 256, sm, st>>>(jobs, radial, cx, cand, cval);
+    for (int pass = 1; pass <= 2; ++pass)
+        k_search1d<<<dim3(ctas, njobs), k1DThreads, sm, st>>>(pass, jobs, radial, cx, cand, cval, best, first,
+                                                              arrive);
 }
 
 void launch_table_search(const TableArgs& a, cudaStream_t st)

@@ -263,8 +263,20 @@ void launch_ctf_res(const float* ctf, int tile, const SearchJob* jobs, int njobs
 // gcf_control.cu: candidate kernel with the state machine in its last blocks
 void launch_eval2d(const EvalArgs& a, int cand_blocks, int max_band_n, cudaStream_t st);
 void launch_init_jobs(const EvalArgs& a, cudaStream_t st);
-void launch_search1d(SearchJob* jobs, int njobs, const float* radial, int cx, float4* cand,
-                     float2* cval, cudaStream_t st);
+// 1D search of the Do2D / Do1D / Refine1D jobs: `ctas` CTAs per job
+// (search1d_ctas); best: njobs * ctas and first: njobs entries of scratch;
+// arrive: njobs zeroed counters (zero again afterwards).
+struct Best1D {
+    float v;
+    int i;
+};
+struct First1D {   // pass 1's best defocus and phase, and the grid points it scored
+    float df, ph;
+    int n;
+};
+int search1d_ctas(int njobs, bool phase, int sms);
+void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, float4* cand,
+                     float2* cval, Best1D* best, First1D* first, int* arrive, cudaStream_t st);
 void launch_shell_select(SearchJob* jobs, int njobs, const float* cc, int cx, int cy,
                          cudaStream_t st);
 // counts (nullable): per job n_cand2d, n_cand1d, n_pairs1d
