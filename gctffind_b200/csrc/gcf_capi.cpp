@@ -224,14 +224,15 @@ struct gcf_ctx {
     DBuf<float> lpfull;
     DBuf<float2> lpcmp;
     DBuf<float> raw, ctf0, ctf, radial, band_spec, cc_res, full;
-    DBuf<int> lowpassed, spec_off, mic_of;
+    DBuf<int> lowpassed, mic_of;
+    DBuf<int2> spec_off;
     DBuf<SearchJob> jobs;
     DBuf<double> sum_ss, ring_sums;
+    DBuf<double2> part, part_grid;
+    DBuf<BestCand> best;
     DBuf<float4> cand;
-    DBuf<float2> cval;
-    DBuf<double2> part;
     DBuf<int> arrive;
-    DBuf<Best1D> best_1d;
+    DBuf<BestCand> best_1d, best_y;
     DBuf<First1D> first_1d;
     DBuf<gcf_result> d_res;
     DBuf<PixOptics> d_optics;
@@ -1026,6 +1027,44 @@ struct SearchPending {
     cudaStream_t st = nullptr;
 };
 
+// Buffers of nj search jobs whose bands hold `tot` pixels in all, at most
+// max_chunks chunks each (any_grid: some job searches the astigmatism grid).
+gcf_status search_buffers(gcf_ctx* ctx, int nj, int tot, int max_chunks, bool any_grid)
+{
+    CK(ctx->jobs.ensure(2 * (size_t)nj));
+    CK(ctx->spec_off.ensure(nj));
+    CK(ctx->band_spec.ensure(std::max(tot, 1)));
+    CK(ctx->sum_ss.ensure(nj));
+    CK(ctx->part.ensure(2 * (size_t)nj * kLineCand * max_chunks));
+    CK(ctx->part_grid.ensure(any_grid ? (size_t)nj * kMaxCand * max_chunks : 1));
+    CK(ctx->best.ensure(2 * (size_t)nj));
+    CK(ctx->cand.ensure((size_t)nj * kMaxCand));
+    CK(ctx->arrive.ensure((size_t)nj * (1 + kMaxCandBlocks)));
+    CK(ctx->best_y.ensure((size_t)nj * kMaxCandBlocks));
+    if (ctx->n_sms == 0) CK(cudaDeviceGetAttribute(&ctx->n_sms, cudaDevAttrMultiProcessorCount, ctx->dev));
+    return GCF_OK;
+}
+
+EvalArgs eval_args(gcf_ctx* ctx, int nj, int max_chunks)
+{
+    EvalArgs a;
+    a.jobs = ctx->jobs.p;
+    a.part = ctx->part.p;
+    a.part_grid = ctx->part_grid.p;
+    a.best = ctx->best.p;
+    a.cand = ctx->cand.p;
+    a.bands = ctx->d_bands.p;
+    a.band_spec = ctx->band_spec.p;
+    a.sum_ss = ctx->sum_ss.p;
+    a.spec_off = ctx->spec_off.p;
+    a.arrive = ctx->arrive.p;
+    a.arrive_y = ctx->arrive.p + nj;
+    a.best_y = ctx->best_y.p;
+    a.max_chunks = max_chunks;
+    a.njobs = nj;
+    return a;
+}
+
 gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, SearchPending& pend)
 {
     int nj = (int)specs.size();
@@ -1036,7 +1075,7 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     int T = ctx->tile, cx = T / 2 + 1;
     size_t cmp_n = (size_t)cx * T;
     std::vector<SearchJob> jh(nj);
-    std::vector<int> soff(nj);
+    std::vector<int2> soff(nj);
     int tot = 0, max_band = 0;
     bool any_full = false, any_grid = false, any_phase = false, any_1d = false, any_phase_1d = false;
     for (int j = 0; j < nj; ++j) {
@@ -1055,6 +1094,7 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
         J.r1d_df = s.r1d_df;
         J.r1d_range = s.r1d_range;
         J.step = STEP_CC0;
+        J.fresh = 1;
         if (J.phase_range_in > 0) any_phase_1d = true;
         if (s.mode >= 2) {
             any_1d = true;
@@ -1069,72 +1109,55 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
             any_grid = true;
             if (J.phase_range_in > 0) any_phase = true;
         }
-        soff[j] = tot;
+        soff[j] = make_int2(tot, slot);
         int bn = ctx->bands[slot]->n;
         tot += bn;
         max_band = std::max(max_band, bn);
     }
     CKS(upload_bands(ctx));
     int max_chunks = std::max(1, (max_band + kEvalChunk - 1) / kEvalChunk);
-    CK(ctx->jobs.ensure(nj));
-    CK(ctx->spec_off.ensure(nj));
-    CK(ctx->band_spec.ensure(std::max(tot, 1)));
-    CK(ctx->sum_ss.ensure(nj));
-    CK(ctx->cand.ensure((size_t)nj * kMaxCand));
-    CK(ctx->cval.ensure((size_t)nj * kMaxCand));
-    CK(ctx->part.ensure((size_t)nj * kMaxCand * max_chunks));
+    CKS(search_buffers(ctx, nj, tot, max_chunks, any_grid));
     CK(ctx->cc_res.ensure((size_t)nj * cx));
     CK(ctx->d_res.ensure(nj));
-    CK(ctx->arrive.ensure(nj));
-    if (ctx->n_sms == 0) CK(cudaDeviceGetAttribute(&ctx->n_sms, cudaDevAttrMultiProcessorCount, ctx->dev));
     const int ctas_1d = search1d_ctas(nj, any_phase_1d, ctx->n_sms);
     CK(ctx->best_1d.ensure((size_t)nj * ctas_1d));
     CK(ctx->first_1d.ensure(nj));
-    CK(cudaMemsetAsync(ctx->arrive.p, 0, nj * sizeof(int), ctx->st));
-    CK(h2d(ctx, ctx->jobs.p, jh.data(), nj * sizeof(SearchJob), ctx->st));
-    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int), ctx->st));
-    launch_band_gather(ctx->ctf.p, (int)cmp_n, ctx->jobs.p, ctx->d_bands.p, ctx->spec_off.p, nj,
+    // Upper bound of non-empty steps: CC0 + astigmatism grid + 19 x 4
+    // refinements; one more launch ends the last of them.  The state buffers
+    // alternate, so that the last launch writes buffer 0.
+    bool any_2d = false;
+    for (const JobSpec& s : specs) any_2d = any_2d || s.mode <= 1;
+    const int steps = any_2d ? 3 + 19 * ((any_grid ? 2 : 0) + 1 + (any_phase ? 1 : 0)) : 0;
+    const int k0 = steps & 1;
+    SearchJob* const jobs0 = ctx->jobs.p + (size_t)k0 * nj;
+    CK(cudaMemsetAsync(ctx->arrive.p, 0, (size_t)nj * (1 + kMaxCandBlocks) * sizeof(int), ctx->st));
+    CK(h2d(ctx, jobs0, jh.data(), nj * sizeof(SearchJob), ctx->st));
+    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int2), ctx->st));
+    launch_band_gather(ctx->ctf.p, (int)cmp_n, jobs0, ctx->d_bands.p, ctx->spec_off.p, nj,
                        ctx->band_spec.p, ctx->sum_ss.p, ctx->st);
     CKL();
     ctx->launches += 1;
-    EvalArgs a;
-    a.jobs = ctx->jobs.p;
-    a.bands = ctx->d_bands.p;
-    a.band_spec = ctx->band_spec.p;
-    a.sum_ss = ctx->sum_ss.p;
-    a.spec_off = ctx->spec_off.p;
-    a.cand = ctx->cand.p;
-    a.cval = ctx->cval.p;
-    a.part = ctx->part.p;
-    a.arrive = ctx->arrive.p;
-    a.max_chunks = max_chunks;
-    a.njobs = nj;
+    const EvalArgs a = eval_args(ctx, nj, max_chunks);
     CK(record_timing(ctx->ev[5], ctx->st));
     if (any_full || any_1d) {
-        launch_search1d(ctx->jobs.p, nj, ctas_1d, ctx->radial.p, cx, ctx->cand.p, ctx->cval.p, ctx->best_1d.p,
-                        ctx->first_1d.p, ctx->arrive.p, ctx->st);
+        launch_search1d(jobs0, nj, ctas_1d, ctx->radial.p, cx, ctx->best_1d.p, ctx->first_1d.p, ctx->arrive.p,
+                        ctx->st);
         CKL();
         ctx->launches += 2;
     }
-    launch_init_jobs(a, ctx->st);   // Refine jobs: pending step CC0
-    CKL();
-    ctx->launches += 1;
     CK(record_timing(ctx->ev[6], ctx->st));
-    // Upper bound of non-empty steps: CC0 + astigmatism grid + 19 x 4 refinements.
-    bool any_2d = false;
-    for (const JobSpec& s : specs) any_2d = any_2d || s.mode <= 1;
-    int pairs = any_2d ? 2 + 19 * ((any_grid ? 2 : 0) + 1 + (any_phase ? 1 : 0)) : 0;
-    // Candidate blocks per (chunk, job) of the line searches (<= 61
-    // candidates, 4 blocks of 16): one block loops over the candidate blocks
-    // it is given, reusing its pixels, so with many jobs fewer y-blocks
-    // (enough for about two waves of 3 CTAs per SM) do the same work without
-    // the blocks that find no candidates and exit.
+    // Candidate blocks per (chunk, job) of the line searches (at most 4
+    // blocks of 16 but for wide phase ranges): one block loops over the
+    // candidate blocks it is given, reusing its pixels, so with many jobs
+    // fewer y-blocks (enough for about four CTAs per SM: 8 jobs 2040 us
+    // against 2164 us with enough for six) do the same work without the
+    // blocks that find no candidates and exit.
     const long long per_y = (long long)nj * max_chunks;
-    const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (2LL * 3 * ctx->n_sms + per_y - 1) / per_y));
-    for (int k = 0; k < pairs; ++k) {
+    const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (4LL * ctx->n_sms + per_y - 1) / per_y));
+    const int last_ends = eval_last_ends(per_y, ctx->n_sms);
+    for (int k = 0; k < steps; ++k) {
         int cb = (k == 0) ? 1 : (k == 1 && any_grid) ? (kMaxCand / kEvalCB + 3) / 4 : line_cb;
-        launch_eval2d(a, cb, max_band, ctx->st);
-        CKL();
+        CK(launch_eval2d(a, k0 + k, cb, max_band, last_ends, ctx->st));
         ctx->launches += 1;
     }
     if (any_2d) {
@@ -1263,7 +1286,7 @@ gcf_status run_fast_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, con
     const int T = ctx->tile, cx = T / 2 + 1;
     const size_t cmp_n = (size_t)cx * T;
     std::vector<SearchJob> jh(nj);
-    std::vector<int> soff(nj);
+    std::vector<int2> soff(nj);
     int tot = 0, max_band = 0;
     for (int j = 0; j < nj; ++j) {
         const JobSpec& sp = specs[j];
@@ -1278,26 +1301,19 @@ gcf_status run_fast_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, con
         J.ext_phase_in = sp.phase_deg;
         J.held_phase = sp.held_phase;
         J.step = STEP_DONE;
-        soff[j] = tot;
+        soff[j] = make_int2(tot, slot);
         const int bn = ctx->bands[slot]->n;
         tot += bn;
         max_band = std::max(max_band, bn);
     }
     CKS(upload_bands(ctx));
     const int max_chunks = std::max(1, (max_band + kEvalChunk - 1) / kEvalChunk);
-    CK(ctx->jobs.ensure(nj));
-    CK(ctx->spec_off.ensure(nj));
-    CK(ctx->band_spec.ensure(std::max(tot, 1)));
-    CK(ctx->sum_ss.ensure(nj));
-    CK(ctx->cand.ensure((size_t)nj * kMaxCand));
-    CK(ctx->cval.ensure((size_t)nj * kMaxCand));
-    CK(ctx->part.ensure((size_t)nj * kMaxCand * max_chunks));
+    CKS(search_buffers(ctx, nj, tot, max_chunks, false));
     CK(ctx->cc_res.ensure((size_t)nj * cx));
     CK(ctx->d_res.ensure(nj));
-    CK(ctx->arrive.ensure(nj));
-    CK(cudaMemsetAsync(ctx->arrive.p, 0, nj * sizeof(int), ctx->st));
+    CK(cudaMemsetAsync(ctx->arrive.p, 0, (size_t)nj * (1 + kMaxCandBlocks) * sizeof(int), ctx->st));
     CK(h2d(ctx, ctx->jobs.p, jh.data(), nj * sizeof(SearchJob), ctx->st));
-    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int), ctx->st));
+    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int2), ctx->st));
     CK(record_timing(ctx->ev[5], ctx->st));
     launch_band_gather(ctx->ctf.p, (int)cmp_n, ctx->jobs.p, ctx->d_bands.p, ctx->spec_off.p, nj, ctx->band_spec.p,
                        ctx->sum_ss.p, ctx->st);
@@ -1375,29 +1391,19 @@ gcf_status run_fast_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, con
     ta.g = g;
     ta.rows = ctx->cRows.p;
     ta.prior = prior;
-    ta.cand = ctx->cand.p;
-    ta.cval = ctx->cval.p;
     launch_table_search(ta, ctx->st);
     CKL();
     ctx->launches += 1;
     CK(record_timing(ctx->ev[6], ctx->st));
     CK(record_timing(ctx->fev[3], ctx->st));
-    EvalArgs a;
-    a.jobs = ctx->jobs.p;
-    a.bands = ctx->d_bands.p;
-    a.band_spec = ctx->band_spec.p;
-    a.sum_ss = ctx->sum_ss.p;
-    a.spec_off = ctx->spec_off.p;
-    a.cand = ctx->cand.p;
-    a.cval = ctx->cval.p;
-    a.part = ctx->part.p;
-    a.arrive = ctx->arrive.p;
-    a.max_chunks = max_chunks;
-    a.njobs = nj;
-    // FP32 re-score + local passes: candidate blocks of 16 (<= 27 per step)
-    for (int k = 0; k < 1 + kLocalPasses; ++k) {
-        launch_eval2d(a, 2, max_band, ctx->st);
-        CKL();
+    const EvalArgs a = eval_args(ctx, nj, max_chunks);
+    // FP32 re-score + local passes: candidate blocks of 16 (<= 27 per step);
+    // the last launch ends the last pass, in buffer 0
+    constexpr int kSteps = 2 + kLocalPasses;
+    static_assert(kSteps % 2 == 0, "the final states land in buffer 0");
+    const int last_ends = eval_last_ends((long long)nj * max_chunks, ctx->n_sms);
+    for (int k = 0; k < kSteps; ++k) {
+        CK(launch_eval2d(a, k, 2, max_band, last_ends, ctx->st));
         ctx->launches += 1;
     }
     CK(record_timing(ctx->fev[4], ctx->st));
@@ -1961,11 +1967,13 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->jobs.release();
     ctx->sum_ss.release();
     ctx->ring_sums.release();
-    ctx->cand.release();
-    ctx->cval.release();
     ctx->part.release();
+    ctx->part_grid.release();
+    ctx->best.release();
+    ctx->cand.release();
     ctx->arrive.release();
     ctx->best_1d.release();
+    ctx->best_y.release();
     ctx->first_1d.release();
     ctx->d_res.release();
     ctx->d_optics.release();

@@ -5,11 +5,10 @@
 // Here the whole control flow lives on the GPU:
 //   k_search1d : radial average -> 1D brute force -> 1D refine -> 2D init,
 //                one CTA per Do2D job (CFindCtf1D::Do1D, FindCTF/CFindCtf1D.cpp:49-111);
-//   k_eval2d   : one step of every job's line search: all pending candidates
-//                against all band pixels, then (last block of each job)
-//                reduce, take the first strict maximum, advance the
-//                CFindDefocus2D::mIterate state machine and write the next
-//                candidate set.
+//   k_eval2d   : one step of every job's line search: reduce the step
+//                before, take the first strict maximum, advance the
+//                CFindDefocus2D::mIterate state machine, and evaluate the
+//                next candidate set against all band pixels.
 // The host only enqueues k_eval2d launches; no value comes back until the
 // search is over.
 //
@@ -262,7 +261,7 @@ __device__ int prepare_step(SearchJob& J, float2* cval)
         if (pmin < 0) pmin = 0.0f;
         if (pmax > 150) pmax = 150.0f;
         int k = 0;
-        for (int i = 0; i < n && k < kMaxCand; ++i) {
+        for (int i = 0; i < n && k < kLineCand; ++i) {
             float ph = J.ext_phase + (i - n / 2) * step;
             if (ph < pmin || ph > pmax) continue;
             cval[k++] = make_float2(ph, 0.0f);
@@ -432,82 +431,67 @@ __device__ ArgMax block_argmax(ArgMax m, ArgMax* sh)
     return r;
 }
 
-__device__ void write_candidates(const SearchJob& J, int n, float4* cand, float2* cval)
-{
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        Cand c = cand_of(J, i, cval);
-        cand[i] = cand_params(c, J.o);
-    }
-}
-
 // ---------------------------------------------------------------------------
-// One block finishes job j's pending line search: reduce the candidates'
-// partial sums in chunk order, take the first strict maximum, advance the
-// CFindDefocus2D::mIterate state machine and write the next candidates.
-__device__ void update_job(int j, SearchJob* __restrict__ jobs, const BandDev* __restrict__ bands,
-                           const double* __restrict__ sum_ss, float4* __restrict__ cand,
-                           float2* __restrict__ cval, const double2* __restrict__ part, int max_chunks)
+// ---------------------------------------------------------------------------
+// Best of the candidates of job j's pending step that lie in the candidate
+// blocks y, y + gy, ... (n of them, counted up to whole blocks; those at or
+// beyond ncand do not exist): sums the chunks' partial sums of each (part:
+// [chunk][pitch], so the threads of a warp read adjacent candidates) and
+// keeps the first strict maximum in index order.  One round takes np (a
+// power of two >= n, at most the block size) candidates; the blockDim / np
+// threads of a candidate share its chunks, each with several loads in flight.
+__device__ ArgMax reduce_candidates(int n, int y, int gy, int ncand, const double2* __restrict__ part, int pitch,
+                                    int nch, double ss, double2* shs, ArgMax* shm, float* cc0)
 {
-    __shared__ SearchJob sJ;
-    __shared__ ArgMax shm[32];
-    __shared__ float s_cc0;
-    __shared__ int s_n;
-    if (threadIdx.x == 0) sJ = jobs[j];
-    __syncthreads();
-    if (sJ.step == STEP_DONE) return;
-    float4* cj = cand + (size_t)j * kMaxCand;
-    float2* vj = cval + (size_t)j * kMaxCand;
-    const int n = sJ.ncand;
-    const BandDev b = bands[sJ.band];
-    const int nch = (b.n + kEvalChunk - 1) / kEvalChunk;
-    const double ss = sum_ss[j];
+    int np = 1;
+    while (np < n && np < kEvalThreads) np <<= 1;
+    const int G = kEvalThreads / np, u = threadIdx.x & (np - 1), q = threadIdx.x / np;
     ArgMax m{(float)-1e20, -1};
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        const double2* p = part + ((size_t)j * kMaxCand + c) * max_chunks;
+    for (int u0 = 0; u0 < n; u0 += np) {
         double cs = 0.0, cc = 0.0;
-        for (int k = 0; k < nch; ++k) {
-            double2 v = p[k];
-            cs += v.x;
-            cc += v.y;
+        const int c = (y + (u0 + u) / kEvalCB * gy) * kEvalCB + (u0 + u) % kEvalCB;
+        const bool have = u0 + u < n && c < ncand;
+        if (have) {
+            const double2* p = part + c;
+#pragma unroll 8
+            for (int k = q; k < nch; k += G) {
+                const double2 v = __ldcg(p + (size_t)k * pitch);
+                cs += v.x;
+                cc += v.y;
+            }
         }
-        double d = sqrt(cc * ss);
-        float ccv = (d == 0.0) ? 0.0f : (float)(cs / d);   // GCC2D mGCalc1D, FindCTF/GCC2D.cu:81-87
-        if (c == 0) s_cc0 = ccv;
-        if (ccv > m.v) m = ArgMax{ccv, c};   // strict, in index order per thread
+        if (G > 1) {   // one round only: np >= n
+            shs[threadIdx.x] = make_double2(cs, cc);
+            __syncthreads();
+            if (q == 0)
+                for (int k = 1; k < G; ++k) {
+                    const double2 v = shs[u + k * np];
+                    cs += v.x;
+                    cc += v.y;
+                }
+        }
+        if (q == 0 && have) {
+            const double d = sqrt(cc * ss);
+            const float ccv = (d == 0.0) ? 0.0f : (float)(cs / d);   // GCC2D mGCalc1D, FindCTF/GCC2D.cu:81-87
+            if (c == 0) *cc0 = ccv;
+            if (ccv > m.v) m = ArgMax{ccv, c};   // strict, in index order per thread
+        }
     }
     __syncthreads();
-    m = block_argmax(m, shm);
-    if (threadIdx.x == 0) {
-        sJ.n_cand2d += n;
-        finish_step(sJ, m.i >= 0 ? m.v : (float)-1e20, m.i, s_cc0, vj);
-        s_n = advance(sJ, vj);
-        sJ.ncand = s_n;
-        jobs[j] = sJ;
-    }
-    __syncthreads();
-    write_candidates(sJ, s_n, cj, vj);
+    return block_argmax(m, shm);
 }
 
-// Fresh jobs: the pending step is CC0 with one candidate (Do2D jobs were
-// set up by k_search1d; 1D-only jobs have nothing to search).
-__global__ void k_init_jobs(SearchJob* __restrict__ jobs, float4* __restrict__ cand, float2* __restrict__ cval)
+// One thread: ends the pending step of J with its best candidate m of n
+// (ended; else it is the search's first step) and prepares the next one.
+__device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m, float cc0, float2* cval)
 {
-    __shared__ SearchJob sJ;
-    __shared__ int s_n;
-    const int j = blockIdx.x;
-    if (threadIdx.x == 0) sJ = jobs[j];
-    __syncthreads();
-    if (sJ.mode >= 2) return;
-    float4* cj = cand + (size_t)j * kMaxCand;
-    float2* vj = cval + (size_t)j * kMaxCand;
-    if (threadIdx.x == 0) {
-        sJ.step = STEP_CC0;
-        s_n = advance(sJ, vj);
-        sJ.ncand = s_n;
-        jobs[j] = sJ;
+    if (ended) {
+        J.n_cand2d += n;
+        if (J.step == STEP_PHASE) prepare_step(J, cval);   // the ended step's phases
+        finish_step(J, m.i >= 0 ? m.v : (float)-1e20, m.i, cc0, cval);
     }
-    __syncthreads();
-    write_candidates(sJ, s_n, cj, vj);
+    J.fresh = 0;
+    J.ncand = advance(J, cval);
 }
 
 // ---------------------------------------------------------------------------
@@ -528,35 +512,56 @@ __global__ void k_init_jobs(SearchJob* __restrict__ jobs, float4* __restrict__ c
 // Grid: x = band chunk (kEvalChunk pixels), y = candidate block (kEvalCB
 // candidates, strided), z = job.  Pixel data stay in registers; candidate
 // parameters come from shared memory; partial sums leave as FP64, one slot
-// per (candidate, chunk).  The last block of a job to finish (an arrival
-// counter, no waiting) runs update_job for it, so one launch is one step of
-// every job's search.  No expression here is contracted differently by
+// per (candidate, chunk).  No expression here is contracted differently by
 // -fmad=false: every multiply-add is an explicit fmaf.  Three CTAs per SM
 // (80 registers, 6 pixels per thread) measured faster than two at 8 pixels
 // per thread: more warps hide the sine's latency better than more
 // independent pixels per warp do.
+//
+// One launch is one step of every job's search; consecutive steps are
+// programmatic dependent launches: a step's CTAs start, and load their pixels
+// (which no step writes), while the step before still runs, and wait for it
+// only then.  The state and the sums pass through two buffers by the parity
+// of the step (jin, pin: the launch before's).  Two ways to end a step:
+//
+//  * few CTAs (last_ends = 0): every CTA of the next launch sums the step's
+//    partial sums (up to kLineCand x chunks), advances its own copy of the
+//    job's state machine and makes its own candidates.  A step of one job is
+//    a chain of latencies, not work: with the job's last CTA ending each
+//    step the line steps of a single search took 13-16 us each and 1-3 us of
+//    launch gap, of which 9000-12000 cycles were the state machine, on an SM
+//    that had last run that code many steps ago.  Run by all CTAs at every
+//    step it stays in their instruction caches: 10 us per step.
+//  * many CTAs (last_ends = 1): the same work in every CTA would cost more
+//    than it saves (96 searches at once: 18.6 ms against 16.1 ms), so the
+//    job's last CTA to finish (an arrival counter, no waiting) ends the step
+//    and writes the next candidates.
+//
+// In both, the astigmatism grid's 2601 candidates are summed by the last CTA
+// of each candidate block y, in parallel over y, not by one CTA.
 __global__ void __launch_bounds__(kEvalThreads, 3)
-k_eval2d(SearchJob* __restrict__ jobs, const BandDev* __restrict__ bands, const float* __restrict__ band_spec,
-         const int* __restrict__ spec_off, const double* __restrict__ sum_ss, float4* __restrict__ cand,
-         float2* __restrict__ cval, double2* __restrict__ part, int max_chunks, int* __restrict__ arrive)
+k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const BandDev* __restrict__ bands,
+         const float* __restrict__ band_spec, const int2* __restrict__ spec_off, const double* __restrict__ sum_ss,
+         const double2* __restrict__ pin, double2* __restrict__ pout, double2* __restrict__ pgrid, int max_chunks,
+         float4* __restrict__ cand, int* __restrict__ arrive, int* __restrict__ arrive_y,
+         BestCand* __restrict__ best_y, const BestCand* __restrict__ best_in,
+         BestCand* __restrict__ best_out, int last_ends)
 {
     __shared__ float4 sq[kEvalCB];
     __shared__ float red[kEvalThreads / 32][2 * kEvalCB];
+    __shared__ double2 shs[kEvalThreads];
+    __shared__ ArgMax shm[32];
+    __shared__ SearchJob sJ;
+    __shared__ float2 s_cval[kLineCand];
+    __shared__ float s_cc0;
     __shared__ int s_last;
     const int j = blockIdx.z;
-    const int ncand = jobs[j].ncand;
-    const int cand_blocks = (ncand + kEvalCB - 1) / kEvalCB;
-    if ((int)blockIdx.y >= cand_blocks) return;
-    // steps whose candidates move one parameter by a fixed step: the mean
-    // defocus, the astigmatism magnitude or the phase (in candidate order),
-    // and the single candidate of CC0
-    const int kind = jobs[j].step;
-    const bool linear = kind == STEP_CC0 || kind == STEP_ASTMAG || kind == STEP_DFMEAN || kind == STEP_PHASE;
-    const BandDev b = bands[jobs[j].band];
+    const int2 so = spec_off[j];   // (offset of the job's band spectrum, band)
+    const BandDev b = bands[so.y];
     const int nchunk = (b.n + kEvalChunk - 1) / kEvalChunk;
     const int p0 = blockIdx.x * kEvalChunk;
     if ((int)blockIdx.x >= max(nchunk, 1)) return;
-    const float* S = band_spec + spec_off[j];
+    const float* S = band_spec + so.x;
     // per pixel: a, d, envelope and -envelope/2, cos 2theta, sin 2theta, spectrum
     float pa[kEvalPPT], pd[kEvalPPT], pe[kEvalPPT], ph[kEvalPPT], pc[kEvalPPT], ps[kEvalPPT], pv[kEvalPPT];
 #pragma unroll
@@ -579,14 +584,58 @@ k_eval2d(SearchJob* __restrict__ jobs, const BandDev* __restrict__ bands, const 
         }
         ph[k] = -0.5f * pe[k];
     }
+    // the step before has ended and its writes are visible; the next step's
+    // CTAs may start
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    constexpr int kJobWords = sizeof(SearchJob) / 4;
+    static_assert(sizeof(SearchJob) % 4 == 0 && kJobWords <= kEvalThreads, "one word of the state per thread");
+    // open: a step of this search is pending; fresh: its first, with no
+    // candidates yet
+    const int* const jw = reinterpret_cast<const int*>(jin + j);
+    int kind = __ldcg(&jin[j].step), ncand = __ldcg(&jin[j].ncand);
+    const bool open = kind != STEP_DONE, fresh = __ldcg(&jin[j].fresh) != 0;
+    if (!last_ends || fresh || !open) {
+        if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = __ldcg(jw + threadIdx.x);
+        __syncthreads();
+        if (open) {
+            ArgMax m{0.0f, -1};
+            if (!fresh && ncand > kLineCand) {   // the launch before chose
+                const float2 q = __ldcg(reinterpret_cast<const float2*>(best_in + j));
+                m = ArgMax{q.x, __float_as_int(q.y)};
+            } else if (!fresh) {
+                m = reduce_candidates(ncand, 0, 1, ncand, pin + (size_t)j * max_chunks * kLineCand, kLineCand, nchunk,
+                                      sum_ss[j], shs, shm, &s_cc0);
+            }
+            if (threadIdx.x == 0) next_step(sJ, !fresh, ncand, m, s_cc0, s_cval);
+            __syncthreads();
+            kind = sJ.step;
+            ncand = sJ.ncand;
+        }
+        if ((!last_ends || !open) && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
+            reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
+        if (kind == STEP_DONE) return;
+    }
+    const int cand_blocks = (ncand + kEvalCB - 1) / kEvalCB;
+    if ((int)blockIdx.y >= cand_blocks) return;
+    // steps whose candidates move one parameter by a fixed step: the mean
+    // defocus, the astigmatism magnitude or the phase (in candidate order),
+    // and the single candidate of CC0
+    const bool linear = kind == STEP_CC0 || kind == STEP_ASTMAG || kind == STEP_DFMEAN || kind == STEP_PHASE;
+    const bool two = ncand > kLineCand;   // a grid: summed in two levels
+    const int pitch = two ? kMaxCand : kLineCand;
+    double2* const pj = (two ? pgrid : pout) + (size_t)j * max_chunks * pitch;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // candidate blocks y, y + gridDim.y, ... so any candidate count is covered
     for (int c0 = blockIdx.y * kEvalCB; c0 < ncand && nchunk > 0; c0 += gridDim.y * kEvalCB) {
         __syncthreads();
         if (threadIdx.x < kEvalCB) {
-            int c = c0 + threadIdx.x;
-            sq[threadIdx.x] =
-                c < ncand ? cand[(size_t)j * kMaxCand + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int c = c0 + threadIdx.x;
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < ncand)
+                q = last_ends && !fresh ? __ldcg(cand + (size_t)j * kMaxCand + c)
+                                        : cand_params(cand_of(sJ, c, s_cval), sJ.o);
+            sq[threadIdx.x] = q;
         }
         __syncthreads();
         float acs[kEvalCB], acc[kEvalCB];
@@ -696,20 +745,57 @@ k_eval2d(SearchJob* __restrict__ jobs, const BandDev* __restrict__ bands, const 
                     s1 += (double)red[w][2 * threadIdx.x];
                     s2 += (double)red[w][2 * threadIdx.x + 1];
                 }
-                part[((size_t)j * kMaxCand + c) * max_chunks + blockIdx.x] = make_double2(s1, s2);
+                pj[(size_t)blockIdx.x * pitch + c] = make_double2(s1, s2);
             }
         }
     }
-    // arrival: the last working block of job j finishes its step
-    const int expected = max(nchunk, 1) * min((int)gridDim.y, cand_blocks);
+    if (!last_ends && ncand <= kLineCand) return;   // summed by the next launch's CTAs
+    // arrival: the last CTA of the job, or of its candidate block y (blocks
+    // y, y + gridDim.y, ...) where there are many candidates
+    const int y = blockIdx.y, gy = gridDim.y, ny = min(gy, cand_blocks), nx = max(nchunk, 1);
+    int* const count = two ? arrive_y + (size_t)j * kMaxCandBlocks + y : arrive + j;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(arrive + j, 1) == expected - 1);
+    if (threadIdx.x == 0) s_last = (atomicAdd(count, 1) == (two ? nx : nx * ny) - 1);
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (threadIdx.x == 0) arrive[j] = 0;
-    update_job(j, jobs, bands, sum_ss, cand, cval, part, max_chunks);
+    if (threadIdx.x == 0) *count = 0;
+    ArgMax m = reduce_candidates(two ? (cand_blocks - y + gy - 1) / gy * kEvalCB : ncand, two ? y : 0, two ? gy : 1, ncand,
+                          pj, pitch, nchunk, sum_ss[j], shs, shm, &s_cc0);
+    if (two) {
+        BestCand* bj = best_y + (size_t)j * kMaxCandBlocks;
+        if (threadIdx.x == 0) {
+            bj[y] = BestCand{m.v, m.i};
+            __threadfence();
+            s_last = (atomicAdd(arrive + j, 1) == ny - 1);
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (threadIdx.x == 0) arrive[j] = 0;
+        m = ArgMax{0.0f, -1};
+        for (int k = threadIdx.x; k < ny; k += kEvalThreads) {
+            const float2 q = __ldcg(reinterpret_cast<const float2*>(bj + k));
+            m = better(m, ArgMax{q.x, __float_as_int(q.y)});
+        }
+        __syncthreads();
+        m = block_argmax(m, shm);
+    }
+    if (!last_ends) {   // a grid: the next launch's CTAs end it with this
+        if (threadIdx.x == 0) best_out[j] = BestCand{m.v, m.i};
+        return;
+    }
+    if (!fresh) {
+        if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = __ldcg(jw + threadIdx.x);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) next_step(sJ, true, ncand, m, s_cc0, s_cval);
+    __syncthreads();
+    if (threadIdx.x < kJobWords)
+        reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
+    for (int c = threadIdx.x; c < sJ.ncand; c += kEvalThreads)
+        cand[(size_t)j * kMaxCand + c] = cand_params(cand_of(sJ, c, s_cval), sJ.o);
 }
 
 // ---------------------------------------------------------------------------
@@ -825,8 +911,7 @@ __device__ ArgMax brute_1d(const Bins1D& B, int lo_bin, int hi_bin, double ss, c
 // the two passes take 21 and 70 us.
 __global__ void __launch_bounds__(k1DThreads)
 k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ radial, int cx,
-           float4* __restrict__ cand, float2* __restrict__ cval, Best1D* __restrict__ best,
-           First1D* __restrict__ first, int* __restrict__ arrive)
+           BestCand* __restrict__ best, First1D* __restrict__ first, int* __restrict__ arrive)
 {
     extern __shared__ unsigned char smem_raw[];
     Bins1D& B = *reinterpret_cast<Bins1D*>(smem_raw);
@@ -890,7 +975,7 @@ k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ rad
     m = block_argmax(m, shm);
     if (gridDim.x > 1) {
         if (threadIdx.x == 0) {
-            best[(size_t)j * gridDim.x + blockIdx.x] = Best1D{m.v, m.i};
+            best[(size_t)j * gridDim.x + blockIdx.x] = BestCand{m.v, m.i};
             __threadfence();
             s_last = (atomicAdd(arrive + j, 1) == (int)gridDim.x - 1);
         }
@@ -900,8 +985,8 @@ k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ rad
         if (threadIdx.x == 0) arrive[j] = 0;
         m = ArgMax{0.0f, -1};
         for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-            const Best1D q = best[(size_t)j * gridDim.x + k];
-            m = better(m, ArgMax{q.v, q.i});
+            const float2 q = __ldcg(reinterpret_cast<const float2*>(best + (size_t)j * gridDim.x + k));
+            m = better(m, ArgMax{q.x, __float_as_int(q.y)});
         }
         __syncthreads();
         m = block_argmax(m, shm);
@@ -916,8 +1001,6 @@ k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ rad
         if (threadIdx.x == 0) first[j] = First1D{b_df, b_ph, g.points()};
         return;
     }
-    float2* vj = cval + (size_t)j * kMaxCand;
-    __shared__ int s_n;
     if (threadIdx.x == 0) {
         const int n1d = f1.n + g.points();
         sJ.n_cand1d += n1d;
@@ -927,7 +1010,6 @@ k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ rad
         sJ.score_1d = b_cc;
         if (sJ.mode >= 2) {   // Do1D / Refine1D alone: no 2D search follows
             sJ.step = STEP_DONE;
-            s_n = 0;
         } else {
             // CFindCtf2D::Do2D + CFindDefocus2D::Setup3/DoIt (FindCTF/CFindCtf2D.cpp:44-53,
             // FindCTF/CFindDefocus2D.cpp:98-124)
@@ -945,13 +1027,11 @@ k_search1d(int pass, SearchJob* __restrict__ jobs, const float* __restrict__ rad
             sJ.ang_range[0] = -90.0f;
             sJ.ang_range[1] = 90.0f;
             sJ.step = STEP_CC0;
-            s_n = advance(sJ, vj);
+            sJ.fresh = 1;
         }
-        sJ.ncand = s_n;
+        sJ.ncand = 0;
         jobs[j] = sJ;
     }
-    __syncthreads();
-    write_candidates(sJ, s_n, cand + (size_t)j * kMaxCand, vj);
 }
 
 // Shell choice of GSpectralCC2D::DoIt (FindCTF/GSpectralCC2D.cu:144-172) and
@@ -1078,7 +1158,7 @@ k_table_search(TableArgs A)
     __shared__ SearchJob sJ;
     __shared__ ArgMax shm[32];
     __shared__ float s_c2[kTabMaxTheta], s_s2[kTabMaxTheta];
-    __shared__ float2 s_cval[kMaxCand];
+    __shared__ float2 s_cval[kLineCand];
     __shared__ float s_cc0;
     __shared__ int s_n;
     __shared__ float s_top[45];
@@ -1226,28 +1306,40 @@ k_table_search(TableArgs A)
         sJ.cc_max = (float)-1e20;
         sJ.iter = 0;
         sJ.step = STEP_RESCORE;
-        s_n = advance(sJ, s_cval);
-        sJ.ncand = s_n;
+        sJ.fresh = 1;
+        sJ.ncand = 0;
         A.jobs[j] = sJ;
     }
-    __syncthreads();
-    write_candidates(sJ, s_n, A.cand + (size_t)j * kMaxCand, A.cval + (size_t)j * kMaxCand);
 }
 
 }  // namespace
 
-void launch_eval2d(const EvalArgs& a, int cand_blocks, int max_band_n, cudaStream_t st)
-{
-    if (a.njobs <= 0 || cand_blocks <= 0 || max_band_n < 0) return;
-    dim3 grid(std::max(1, (max_band_n + kEvalChunk - 1) / kEvalChunk), cand_blocks, a.njobs);
-    k_eval2d<<<grid, kEvalThreads, 0, st>>>(a.jobs, a.bands, a.band_spec, a.spec_off, a.sum_ss, a.cand,
-                                            a.cval, a.part, a.max_chunks, a.arrive);
-}
+// 1 search (41 CTAs per candidate block): 775 us with every CTA ending the
+// step before, 860 us with the last CTA ending each; 2 (82 CTAs) 995 and
+// 1040; 4 (164 CTAs) 1454 and 1369; 8 (328 CTAs) 2375 and 2042.
+int eval_last_ends(long long ctas, int sms) { return ctas > sms ? 1 : 0; }
 
-void launch_init_jobs(const EvalArgs& a, cudaStream_t st)
+cudaError_t launch_eval2d(const EvalArgs& a, int k, int cand_blocks, int max_band_n, int last_ends,
+                          cudaStream_t st)
 {
-    if (a.njobs <= 0) return;
-    k_init_jobs<<<a.njobs, 256, 0, st>>>(a.jobs, a.cand, a.cval);
+    if (a.njobs <= 0 || cand_blocks <= 0 || max_band_n < 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::max(1, (max_band_n + kEvalChunk - 1) / kEvalChunk), std::min(cand_blocks, kMaxCandBlocks),
+                       a.njobs);
+    cfg.blockDim = dim3(kEvalThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const int in = k & 1, out = in ^ 1;
+    const size_t np = (size_t)a.njobs * a.max_chunks * kLineCand;
+    return cudaLaunchKernelEx(&cfg, k_eval2d, (const SearchJob*)(a.jobs + (size_t)in * a.njobs),
+                              a.jobs + (size_t)out * a.njobs, a.bands, a.band_spec, a.spec_off, a.sum_ss,
+                              (const double2*)(a.part + in * np), a.part + out * np, a.part_grid, a.max_chunks,
+                              a.cand, a.arrive, a.arrive_y, a.best_y, (const BestCand*)(a.best + (size_t)in * a.njobs),
+                              a.best + (size_t)out * a.njobs, last_ends);
 }
 
 int search1d_ctas(int njobs, bool phase, int sms)
@@ -1259,14 +1351,13 @@ int search1d_ctas(int njobs, bool phase, int sms)
     return std::max(1, std::min(want, 4 * sms / std::max(njobs, 1)));
 }
 
-void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, float4* cand,
-                     float2* cval, Best1D* best, First1D* first, int* arrive, cudaStream_t st)
+void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, BestCand* best,
+                     First1D* first, int* arrive, cudaStream_t st)
 {
     if (njobs <= 0) return;
     size_t sm = sizeof(Bins1D);   // 16.4 KB, below the default dynamic limit
     for (int pass = 1; pass <= 2; ++pass)
-        k_search1d<<<dim3(ctas, njobs), k1DThreads, sm, st>>>(pass, jobs, radial, cx, cand, cval, best, first,
-                                                              arrive);
+        k_search1d<<<dim3(ctas, njobs), k1DThreads, sm, st>>>(pass, jobs, radial, cx, best, first, arrive);
 }
 
 void launch_table_search(const TableArgs& a, cudaStream_t st)

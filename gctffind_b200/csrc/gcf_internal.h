@@ -75,6 +75,9 @@ constexpr int kEvalThreads = 256;     // threads of the candidate kernel
 constexpr int kEvalPPT = 6;           // band pixels per thread per chunk
 constexpr int kEvalChunk = kEvalThreads * kEvalPPT;
 constexpr int kEvalCB = 16;           // candidates per CTA
+constexpr int kLineCand = 160;        // >= the candidates of any step but the grid: at most
+                                      // 151 phases (0 to 150 degrees by at least one, or 61)
+constexpr int kMaxCandBlocks = 64;    // grid.y of a search step at most
 constexpr int kMax1DBins = 1025;      // tile <= 2048
 
 // Search step kinds (CFindDefocus2D::mIterate, FindCTF/CFindDefocus2D.cpp:153-183)
@@ -111,7 +114,7 @@ struct SearchJob {
     int band;           // band-table slot
     int mode;           // 0 = Do2D (after the 1D search), 1 = Refine, 2 = Do1D, 3 = Refine1D,
                         // 4 = contraction search (table search, then the FP32 finish)
-    int pad0;
+    int fresh;          // the pending step has no candidates yet (nothing to finish)
     PixOptics o;
     float phase_range_in;   // CFindCtfBase::m_fPhaseRange (Do2D)
     float ext_phase_in;     // CFindCtfBase::m_fExtPhase   (Do2D)
@@ -151,6 +154,12 @@ struct SearchJob {
     int pad3;
 };
 
+// Best score and its index (a CTA's share of a search step).
+struct __align__(8) BestCand {
+    float v;
+    int i;
+};
+
 // Per-band device pointers (structure of arrays).
 struct BandDev {
     int n;
@@ -166,15 +175,21 @@ struct BandDev {
 
 // Arguments of the 2D candidate kernels.
 struct EvalArgs {
-    SearchJob* jobs;
+    // two buffers each, by the parity of the step: the state and sums that
+    // the launch before wrote, and those that this one writes
+    SearchJob* jobs;            // [2][job]
+    double2* part;              // [2][job][max_chunks][kLineCand] (sum CS, sum CC)
+    double2* part_grid;         // [job][max_chunks][kMaxCand] the same of the astigmatism grid
+    float4* cand;               // [job][kMaxCand] candidates made by the step's last CTA:
+                                // (mean_px, sig*cos2a, sig*sin2a, phase/pi)
+    BestCand* best;             // [2][job] best candidate of a grid
     const BandDev* bands;
     const float* band_spec;     // [job][band pixels] spectrum gathered in band order
     const double* sum_ss;       // [job] sum of S^2 over the band
-    const int* spec_off;        // [job] offset of the job's band spectrum
-    float4* cand;               // [job][kMaxCand] (mean_px, sig*cos2a, sig*sin2a, phase/pi)
-    float2* cval;               // [job][kMaxCand] searched parameter values
-    double2* part;              // [job][kMaxCand][max_chunks] (sum CS, sum CC)
-    int* arrive;                // [job] blocks of the current step done (0 between steps)
+    const int2* spec_off;       // [job] (offset of the job's band spectrum, its band)
+    int* arrive;                // [job] candidate blocks of the step summed (0 between steps)
+    int* arrive_y;              // [job][kMaxCandBlocks] CTAs of a candidate block done (0 between steps)
+    BestCand* best_y;           // [job][kMaxCandBlocks] best candidate of each candidate block
     int max_chunks;
     int njobs;
 };
@@ -251,7 +266,7 @@ void launch_lp_extract(const float* ctf0, const float* full, int tile, int nmic,
 void launch_radial(const float* spect, int tile, int nmic, const int* off, const int* pix,
                    float* radial, cudaStream_t st);
 void launch_band_gather(const float* ctf, int cmp_n, const SearchJob* jobs, const BandDev* bands,
-                        const int* spec_off, int njobs, float* band_spec, double* sum_ss,
+                        const int2* spec_off, int njobs, float* band_spec, double* sum_ss,
                         cudaStream_t st);
 void launch_full_spectrum(const float* ctf, int tile, int nmic, const int* mic_of,
                           const gcf_result* res, const PixOptics* o, const double* moments,
@@ -260,23 +275,27 @@ void launch_ctf_res(const float* ctf, int tile, const SearchJob* jobs, int njobs
                     const int* ring_pix, const double2* ring_geo, double* ring_sums, float* cc,
                     cudaStream_t st);
 
-// gcf_control.cu: candidate kernel with the state machine in its last blocks
-void launch_eval2d(const EvalArgs& a, int cand_blocks, int max_band_n, cudaStream_t st);
-void launch_init_jobs(const EvalArgs& a, cudaStream_t st);
+// gcf_control.cu: step k of every job's search: ends step k - 1 and
+// evaluates the next candidates, cand_blocks candidate blocks at a time.
+// Programmatically dependent on the launch before it on st: that launch may
+// still run when this step's CTAs load what no step writes (bands,
+// band_spec, spec_off).  The launch after the last step ends it.
+cudaError_t launch_eval2d(const EvalArgs& a, int k, int cand_blocks, int max_band_n, int last_ends,
+                          cudaStream_t st);
+// Whether the last CTA of a step ends it and makes the next candidates (else
+// every CTA of the next step does), for steps of `ctas` (chunk, job) pairs;
+// the same for all steps of a search.
+int eval_last_ends(long long ctas, int sms);
 // 1D search of the Do2D / Do1D / Refine1D jobs: `ctas` CTAs per job
 // (search1d_ctas); best: njobs * ctas and first: njobs entries of scratch;
 // arrive: njobs zeroed counters (zero again afterwards).
-struct Best1D {
-    float v;
-    int i;
-};
 struct First1D {   // pass 1's best defocus and phase, and the grid points it scored
     float df, ph;
     int n;
 };
 int search1d_ctas(int njobs, bool phase, int sms);
-void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, float4* cand,
-                     float2* cval, Best1D* best, First1D* first, int* arrive, cudaStream_t st);
+void launch_search1d(SearchJob* jobs, int njobs, int ctas, const float* radial, int cx, BestCand* best,
+                     First1D* first, int* arrive, cudaStream_t st);
 void launch_shell_select(SearchJob* jobs, int njobs, const float* cc, int cx, int cy,
                          cudaStream_t st);
 // counts (nullable): per job n_cand2d, n_cand1d, n_pairs1d
@@ -373,8 +392,6 @@ struct TableArgs {
     PolarGrid g;
     const int2* rows;        // [njobs] rows computed for each job
     const float4* prior;     // [njobs] (mean A, ratio, angle deg, window scale) or null
-    float4* cand;
-    float2* cval;
 };
 void launch_table_search(const TableArgs& a, cudaStream_t st);
 // Seeded uniform fills (autotuner trial operands): floats in [lo, hi), BF16 in [-1, 1).

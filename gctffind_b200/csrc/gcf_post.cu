@@ -281,7 +281,7 @@ __global__ void k_radial(const float* __restrict__ spect, int cmp_n, int cx,
 // Spectrum of each job gathered in band order, and its sum of squares.
 __global__ void k_band_gather(const float* __restrict__ ctf, int cmp_n,
                               const SearchJob* __restrict__ jobs, const BandDev* __restrict__ bands,
-                              const int* __restrict__ spec_off, float* __restrict__ band_spec,
+                              const int2* __restrict__ spec_off, float* __restrict__ band_spec,
                               double* __restrict__ sum_ss)
 {
     __shared__ double sh[32];
@@ -289,7 +289,7 @@ __global__ void k_band_gather(const float* __restrict__ ctf, int cmp_n,
     const SearchJob& jb = jobs[j];
     const BandDev& b = bands[jb.band];
     const float* src = ctf + (size_t)jb.mic * cmp_n;
-    float* dst = band_spec + spec_off[j];
+    float* dst = band_spec + spec_off[j].x;
     double v[1] = {0.0};
     const int S = blockDim.x;
     int k = threadIdx.x;
@@ -514,7 +514,7 @@ void launch_radial(const float* spect, int tile, int nmic, const int* off, const
 }
 
 void launch_band_gather(const float* ctf, int cmp_n, const SearchJob* jobs, const BandDev* bands,
-                        const int* spec_off, int njobs, float* band_spec, double* sum_ss,
+                        const int2* spec_off, int njobs, float* band_spec, double* sum_ss,
                         cudaStream_t st)
 {
     if (njobs <= 0) return;
