@@ -219,7 +219,8 @@ struct gcf_ctx {
     DBuf<float> rs_src;   // an aligned copy of a device image cuFFT cannot read in place
     DBuf<__nv_bfloat16> rsg_bf;   // scratch of the tensor-core rescale (gcf_rsgemm.cu)
     DBuf<float> rsg_f;
-    DBuf<int> rsg_err;            // its products' bounded-wait flag, checked when results are read
+    DBuf<int> dev_err;            // bounded-wait flag of the tile kernel and the tensor-core
+                                  // rescale, checked when results are read
     DBuf<double> acc, hsum, moments, moments2, tile_sums;
     DBuf<float> lpfull;
     DBuf<float2> lpcmp;
@@ -510,6 +511,8 @@ gcf_status build_tile_tables(gcf_ctx* ctx)
     }
     CK(ctx->tw512.ensure(T));
     CK(cudaMemcpy(ctx->tw512.p, tw.data(), T * sizeof(float2), cudaMemcpyHostToDevice));
+    CK(ctx->dev_err.ensure(1));
+    CK(cudaMemset(ctx->dev_err.p, 0, sizeof(int)));
     // A copy from pageable memory may return before its DMA lands, and the
     // context's streams are non-blocking (not ordered after these copies):
     // wait for the tables once, at creation.
@@ -869,7 +872,7 @@ gcf_status fused_launch(gcf_ctx* ctx, int m0, int m1, float* raw_out, cudaStream
     if (solo) CKS(solo_setup(ctx, &sl));
     CK(launch_fused(ctx->f_desc.p, ctx->f_bsum_ptr.p, max_blocks, ctx->f_items.p + first[m0], ni, ctx->f_first.p,
                     ctx->f_inv.p, m0, m1 - m0, ctx->taper.p, ctx->tw512.p, ctx->f_partial.p, raw_out,
-                    ctx->f_next.p + m0, ncl, ctx->fused_shape, st, e0, e1, solo ? &sl : nullptr));
+                    ctx->f_next.p + m0, ctx->dev_err.p, ncl, ctx->fused_shape, st, e0, e1, solo ? &sl : nullptr));
     ctx->launches += (solo && sl.n > 0 && ni > ncl) ? 4 : 3;
     return GCF_OK;
 }
@@ -1180,14 +1183,14 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
 }
 
 // Reads back the results of an enqueued search (waits for it on the host).
-// The tensor-core rescale's flag, read back with a call's results: a
-// bounded wait of its products gave up (the flag is cleared for the next
-// call).
-gcf_status check_rescale_gemm(gcf_ctx* ctx, int flag)
+// The device flag of bounded waits, read back with a call's results: a wait
+// of the tile kernel or of the rescale's products gave up (the flag is
+// cleared for the next call).
+gcf_status check_dev_err(gcf_ctx* ctx, int flag)
 {
     if (!flag) return GCF_OK;
-    CK(cudaMemset(ctx->rsg_err.p, 0, sizeof(int)));
-    return fail(ctx, GCF_ERR_TIMEOUT, "tensor-core rescale product: a bounded wait gave up");
+    CK(cudaMemset(ctx->dev_err.p, 0, sizeof(int)));
+    return fail(ctx, GCF_ERR_TIMEOUT, "tile spectrum or tensor-core rescale: a bounded wait gave up");
 }
 
 gcf_status run_search_collect(gcf_ctx* ctx, const SearchPending& pend, std::vector<gcf_result>& out)
@@ -1198,11 +1201,10 @@ gcf_status run_search_collect(gcf_ctx* ctx, const SearchPending& pend, std::vect
     CK(cudaMemcpyAsync(out.data(), ctx->d_res.p, nj * sizeof(gcf_result), cudaMemcpyDeviceToHost, pend.st));
     std::vector<int> cnt(3 * (size_t)nj);
     CK(cudaMemcpyAsync(cnt.data(), ctx->d_counts.p, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, pend.st));
-    int rs_err = 0;
-    if (ctx->rsg_err.p)
-        CK(cudaMemcpyAsync(&rs_err, ctx->rsg_err.p, sizeof(int), cudaMemcpyDeviceToHost, pend.st));
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, pend.st));
     CK(cudaStreamSynchronize(pend.st));
-    CKS(check_rescale_gemm(ctx, rs_err));
+    CKS(check_dev_err(ctx, flag));
     for (int j = 0; j < nj; ++j) {
         const long long n2 = cnt[3 * j], n1 = cnt[3 * j + 1], p1 = cnt[3 * j + 2];
         ctx->search_counts[0] += n2;
@@ -1646,11 +1648,7 @@ gcf_status rescale_device(gcf_ctx* ctx, const float* img, int w, int h, float px
         const RescaleGemmLayout L = rescale_gemm_layout(w, h, nw, nh);
         CK(ctx->rsg_bf.ensure((size_t)L.bf16_elems));
         CK(ctx->rsg_f.ensure((size_t)L.f32_elems));
-        if (!ctx->rsg_err.p) {
-            CK(ctx->rsg_err.ensure(1));
-            CK(cudaMemset(ctx->rsg_err.p, 0, sizeof(int)));
-        }
-        CK(launch_rescale_gemm(img, w, w, h, nw, nh, ctx->rsg_bf.p, ctx->rsg_f.p, ctx->rsg_err.p, out, ctx->st));
+        CK(launch_rescale_gemm(img, w, w, h, nw, nh, ctx->rsg_bf.p, ctx->rsg_f.p, ctx->dev_err.p, out, ctx->st));
         ctx->launches += 5;
         return GCF_OK;
     }
@@ -1946,7 +1944,7 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->rs_src.release();
     ctx->rsg_bf.release();
     ctx->rsg_f.release();
-    ctx->rsg_err.release();
+    ctx->dev_err.release();
     ctx->acc.release();
     ctx->tile_sums.release();
     ctx->hsum.release();
@@ -2096,11 +2094,10 @@ gcf_status gcf_rescale(gcf_ctx* ctx, const float* img, int w, int h, float px, i
         CK(cudaMemcpy2DAsync(host_out, nw * sizeof(float), d, w * sizeof(float),
                              nw * sizeof(float), nh, cudaMemcpyDeviceToHost, ctx->st));
     }
-    int rs_err = 0;
-    if (ctx->rsg_err.p)
-        CK(cudaMemcpyAsync(&rs_err, ctx->rsg_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    return check_rescale_gemm(ctx, rs_err);
+    return check_dev_err(ctx, flag);
 }
 
 gcf_status gcf_set_fused_shape(gcf_ctx* ctx, int shape)
@@ -2145,9 +2142,11 @@ gcf_status gcf_gen_half_spectrum(gcf_ctx* ctx, const float* img, int pitch, int 
     std::vector<MicImage> mics(1);
     mics[0] = MicImage{d, ctx->img_w, ctx->img_h, pitch, ctx->optics.pixel_size};
     CKS(spectra(ctx, mics));
-    int lp = 0;
+    int lp = 0, flag = 0;
     CK(cudaMemcpyAsync(&lp, ctx->lowpassed.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&flag, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    CKS(check_dev_err(ctx, flag));
     ctx->cur_lowpassed = lp;
     ctx->have_spectrum = true;
     return GCF_OK;

@@ -18,6 +18,10 @@
 //           columns share one complex FFT;
 //   |F|     amplitudes (DC moved to row 256) accumulate in registers across
 //           all tiles of a work item and are written once.
+// That is the one-line kernel, k_fused_spectrum, whose shapes the autotuner
+// times and a caller can ask for; the default is k_fused_spectrum_pair, the
+// same work on 8-CTA clusters with two lines per warp, the taper and the sums
+// in tensor memory and the rows' bins exchanged by bulk copies.
 // With CL = 16 the column buffer is double-buffered, so one cluster barrier
 // per tile separates writers from readers.  Beside the cluster launch,
 // k_fused_spectrum_solo runs one CTA on each SM that the clusters leave free
@@ -167,6 +171,157 @@ __device__ __forceinline__ void fft512_warp(float2 (&v)[16], float2* scr, const 
     __syncwarp();
 }
 
+// cmul and amp as the one-line kernels compile them (where the compiler
+// contracts a product into the sum is its choice, so it is pinned here):
+// the two kernels' spectra are the same bits.
+__device__ __forceinline__ float2 cmul_pinned(float2 a, float2 b)
+{
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ float amp_xy(float x, float y)
+{
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(__fmaf_rn(x, x, __fmul_rn(y, y))));
+    return r;
+}
+
+// Two 512-point forward FFTs held by one warp, line h on the lanes of parity
+// h: lane 2a + h holds x[32 j + 2a] of its line in e[j] and x[32 j + 2a + 1]
+// in o[j] on entry, X[a + 16 k] in e[P16(k)] and X[a + 16 k + 256] in
+// o[P16(k)] on return.  Every operation on a line is fft512_warp's (radix 16,
+// twiddles, radix 16 over the even and odd l, radix 2), so the values are the
+// same bits; what changes is where they live.  A lane holds whole 32-point
+// second stages, so the radix 2 needs no lane exchange (32 shuffles and 32
+// selects per line less), pairs of neighbours move as 16-byte accesses (half
+// the shared-memory instructions), and two lines per warp give the scheduler
+// twice the independent work.  scr: line h's 256 float4; row k1 keeps its
+// 16-byte chunk c at c ^ k1 ^ 4 h, so that neither side of the transpose has
+// bank conflicts without padding.  tw4[k1 * 16 + a] = (exp(-2 pi i 2a k1 / 512),
+// exp(-2 pi i (2a + 1) k1 / 512)).  between(0..3) runs at four points of the
+// transform: the caller spreads its global loads over them (32 loads of 256
+// bytes in a row stall a warp for 1000 cycles in the load queue).
+template <class F>
+__device__ __forceinline__ void fft512_pair(float2 (&e)[16], float2 (&o)[16], float4* scr, const float4* tw4,
+                                            int lane, F between)
+{
+    const int a = lane >> 1, ax = a ^ ((lane & 1) << 2);
+    between(0);
+    dft16(e);
+    between(1);
+    dft16(o);
+    between(2);
+#pragma unroll
+    for (int k1 = 1; k1 < 16; ++k1) {
+        const float4 t = tw4[k1 * 16 + a];
+        e[P16(k1)] = cmul_pinned(e[P16(k1)], make_float2(t.x, t.y));
+        o[P16(k1)] = cmul_pinned(o[P16(k1)], make_float2(t.z, t.w));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k1 = 0; k1 < 16; ++k1)
+        scr[k1 * 16 + (ax ^ k1)] = make_float4(e[P16(k1)].x, e[P16(k1)].y, o[P16(k1)].x, o[P16(k1)].y);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const float4 z = scr[a * 16 + (q ^ ax)];
+        e[q] = make_float2(z.x, z.y);
+        o[q] = make_float2(z.z, z.w);
+    }
+    between(3);
+    dft16(e);
+    dft16(o);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const float2 u = cmul_k(o[P16(k)], c_tw32[k]), E = e[P16(k)];
+        e[P16(k)] = cadd(E, u);
+        o[P16(k)] = csub(E, u);
+    }
+}
+
+// Two adjacent samples of a row; v2: the row is 8-byte aligned at even x.
+__device__ __forceinline__ float2 row2(const float* p, bool v2)
+{
+    float2 r;
+    if (v2)
+        asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    else
+        r = make_float2(__ldg(p), __ldg(p + 1));
+    return r;
+}
+
+// The split of one FFT of two real rows (fft512_pair's output z, rows A + i B)
+// into twice the rows' bins K = a + 16 kk, kk < 16: f(kk, (2 A, 2 B)), with the
+// real DC and Nyquist bins of both rows packed at K = 0.  The partner Z[512 - K]
+// of lane a is lane 16 - a's; for a = 0 its own, one index on.
+template <class F>
+__device__ __forceinline__ void split_rows(const float2 (&e)[16], const float2 (&o)[16], int lane, F f)
+{
+    const int a = lane >> 1, from = (lane & 1) | ((16 - a) & 15) << 1;
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+        const float2 zk = e[P16(kk)];
+        float2 s = o[P16(15 - kk)];
+        if (a == 0) s = kk ? o[P16((16 - kk) & 15)] : zk;
+        float2 zn;
+        zn.x = __shfl_sync(0xffffffffu, s.x, from);
+        zn.y = __shfl_sync(0xffffffffu, s.y, from);
+        // twice the two rows' bins (the 1/2 of the split is applied once,
+        // exactly, to the averaged spectrum in k_item_reduce)
+        float4 AB = make_float4(zk.x + zn.x, zk.y - zn.y, zk.y + zn.y, zn.x - zk.x);
+        if (kk == 0 && a == 0) {
+            const float2 zh = o[P16(0)];
+            AB = make_float4(2.0f * zk.x, 2.0f * zh.x, 2.0f * zk.y, 2.0f * zh.y);
+        }
+        f(kk, AB);
+    }
+}
+
+// |F| of the packed column (0, 256) of a tile, on the even lanes: kx = 0 is
+// added to acc, kx = 256 to accN; the odd lanes' column is an ordinary one.
+// Both columns are real lines' transforms, so |F[512 - ky]| = |F[ky]| bit for
+// bit: per tile only ky = a + 16 kk <= 256 are added, and mirror_column fills
+// in the others when the item ends.
+__device__ __forceinline__ void packed_column(const float2 (&e)[16], const float2 (&o)[16], int lane, float* accN,
+                                              float (&acc)[32])
+{
+    const int a = lane >> 1, from = (lane & 1) | ((16 - a) & 15) << 1;
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int kk = 0; kk < 17; ++kk) {
+        const float2 zk = kk < 16 ? e[P16(kk & 15)] : o[P16(0)];
+        float2 s = kk < 16 ? o[P16((15 - kk) & 15)] : e[P16(15)];
+        if (a == 0) s = kk == 0 ? e[P16(0)] : o[P16((16 - kk) & 15)];
+        float2 zn;
+        zn.x = __shfl_sync(0xffffffffu, s.x, from);
+        zn.y = __shfl_sync(0xffffffffu, s.y, from);
+        if (odd) {
+            acc[kk] += amp_xy(zk.x, zk.y);
+        } else if (kk < 16 || a == 0) {
+            float ax = 0.5f * (zk.x + zn.x), ay = 0.5f * (zk.y - zn.y);
+            float bx = 0.5f * (zk.y + zn.y), by = -0.5f * (zk.x - zn.x);
+            acc[kk] += amp_xy(ax, ay);
+            accN[a + 16 * kk] += amp_xy(by, bx);
+        }
+    }
+#pragma unroll
+    for (int kk = 17; kk < 32; ++kk) {
+        const float2 zk = o[P16(kk & 15)];
+        if (odd) acc[kk] += amp_xy(zk.x, zk.y);
+    }
+}
+
+// The bins ky > 256 of kx = 0 from their mirrors 512 - ky (lane 16 - a's, or
+// its own for a = 0).
+__device__ __forceinline__ void mirror_column(int lane, float (&acc)[32])
+{
+    const int a = lane >> 1, from = (lane & 1) | ((16 - a) & 15) << 1;
+#pragma unroll
+    for (int kk = 16; kk < 32; ++kk) {
+        const float s = __shfl_sync(0xffffffffu, a == 0 ? acc[32 - kk] : acc[31 - kk], from);
+        if ((lane & 1) == 0 && (kk > 16 || a > 0)) acc[kk] = s;
+    }
+}
+
 struct FusedTab {
     const float* img;
     const double* bsum;   // sums of the stride x stride blocks, [nty + 1][ntx + 1]
@@ -275,7 +430,6 @@ struct FusedShape {
     static_assert(R % 32 == 0 && PW >= 1 && NR >= 1 && R / 2 == PW * NW && C == NR * NW && C <= 32, "shape");
 };
 using Shape16 = FusedShape<16, 16, true>;         // 16-CTA clusters, 512 threads
-using Shape8 = FusedShape<8, 8, false>;           // 8-CTA clusters, 256 threads
 using Shape8W16 = FusedShape<8, 16, false, false>;  // 8-CTA clusters, 512 threads, 128 registers
 // 16-CTA clusters of 256 threads at <= 128 registers and 107 KB of shared
 // memory: two CTAs (of different clusters, or of one) per SM, so one CTA's
@@ -489,24 +643,427 @@ k_fused_spectrum(const FusedTab* __restrict__ imgs, const int4* __restrict__ ite
     cluster.sync();   // keep shared memory alive until every peer is done
 }
 
+// ---- the same with two lines per warp ----------------------------------------
+// k_fused_spectrum's work on 8-CTA clusters of 8 warps, with every FFT from
+// fft512_pair: a warp transforms four rows (two row pairs), then two columns,
+// at a time.  Values, splits and the order of every addition are the same, so
+// the spectra are the same bits.
+//
+// Bound: instruction issue and latency at 8 warps per SM, and the 64 bytes per
+// clock of the exchange between SMs.  The one-line kernel issued on 35 % of
+// the cycles, mostly waiting for shared memory, shuffles and their queue.  Per
+// 512 x 512 tile and cluster: 16.3 us one line per warp (its 8 x 8 shape), 17.8
+// two lines, 16.0 with the taper and the sums in tensor memory, 13.3 with the
+// bulk copies and the split barrier, 11.8 with the rows half a tile ahead; a
+// launch over 41 micrographs of 4096 x 4096 7.99 -> 6.18 ms.
+//
+// Tensor memory (256 KB per SM, no matrix product here needs it) holds what
+// would not fit in registers or shared memory:
+//  * the taper of the CTA's 64 rows (128 KB; a CTA keeps its rank, so it is
+//    loaded once per launch), which otherwise doubles the tile's L2 reads and
+//    stalls each round for their latency;
+//  * the item's |F| sums (64 KB), whose 64 registers per thread hold rows in
+//    flight instead;
+//  * the first 32 of the next tile's 64 rows, parked while the other 32 come
+//    in (64 KB): all of a tile's rows are read half a tile ahead.
+// Every warp only touches its own lanes and columns, so no barrier is needed.
+//
+// Exchange: a warp stages its four rows' bins in its transpose scratch as one
+// 1 KB block per destination CTA ([column][4 rows]) and eight lanes issue one
+// bulk copy each to their CTA's column buffer; the copies signal an mbarrier
+// there, which the column transforms wait for (bounded).  16-byte stores into
+// the peers' memory, in the same order from every warp, kept the store queue
+// full and needed a releasing cluster barrier per tile (a quarter of the
+// warps' time in both).  The barrier that says "the column buffers have been
+// read" is arrived at after a tile's last column loads and waited for after
+// the next tile's first row transforms.
+template <int CL_, int NW_>
+struct PairShape {
+    static constexpr int CL = CL_;                  // CTAs per cluster
+    static constexpr int NW = NW_;                  // warps per CTA
+    static constexpr int THR = 32 * NW;
+    static constexpr int MINB = 8 / NW;             // CTAs per SM
+    static constexpr int R = FT / CL;               // tile rows per CTA
+    static constexpr int C = FT / 2 / CL;           // frequency columns per CTA
+    static constexpr int BLOCK = C * 4;             // float2 of a block: 4 rows of every column of a CTA
+    static constexpr int ROUNDS = C / (2 * NW);     // dual FFTs per warp, phase and tile
+    static constexpr size_t BUF = (size_t)C * FT * sizeof(float2);
+    static constexpr size_t SCR = (size_t)NW * 2 * FT * sizeof(float2);
+    static constexpr size_t SMEM = BUF + SCR + 16 * 32 * sizeof(float2) + FT * sizeof(float);
+    // tensor-memory columns: per group of four warps (one per lane quarter)
+    // the taper of each round (two rows of 32 values per lane), the sums, the
+    // parked rows
+    static constexpr int TM_TAPER = 64 * ROUNDS, TM_ACC = 32 * ROUNDS, TM_PARK = 64;
+    static constexpr int TM_ACC0 = NW / 4 * TM_TAPER, TM_PARK0 = TM_ACC0 + NW / 4 * TM_ACC;
+    static constexpr int TM_COLS = 512 / MINB;
+    static_assert(ROUNDS == 2 && R == 4 * NW * ROUNDS && NW % 4 == 0 && CL <= 16, "shape");
+    static_assert(TM_PARK0 + NW / 4 * TM_PARK <= TM_COLS, "tensor memory");
+};
+using Pair8 = PairShape<8, 8>;
+
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Waits for the mbarrier phase of the given parity, about a second at most.
+__device__ bool wait_phase(uint32_t bar, uint32_t parity)
+{
+    unsigned long long t0 = 0;
+    for (uint32_t it = 0;; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((it & 63) == 63) {
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            if (now - t0 > 1000000000ull) return false;
+        }
+    }
+}
+
+// 32 values per lane between registers and tensor memory (the warp's lane
+// quarter, 32 columns from addr); a get waits for the warp's earlier puts.
+__device__ __forceinline__ void tmem_get32(uint32_t addr, float (&v)[32])
+{
+    asm volatile(
+        "tcgen05.wait::st.sync.aligned;\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+          "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+          "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(addr));
+}
+__device__ __forceinline__ void tmem_put32(uint32_t addr, const float (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(addr),
+        "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]),
+        "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]),
+        "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31]));
+}
+
+template <class S>
+__global__ void __launch_bounds__(S::THR, S::MINB)
+k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict__ items, int nitems,
+                      const float* __restrict__ taper, const float2* __restrict__ twg,
+                      float* __restrict__ partial, unsigned long long* __restrict__ next_item, int* __restrict__ err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2* colbuf = reinterpret_cast<float2*>(smem);
+    float4* scr_all = reinterpret_cast<float4*>(smem + S::BUF);
+    float2* twl = reinterpret_cast<float2*>(smem + S::BUF + S::SCR);
+    float* accN = reinterpret_cast<float*>(twl + 16 * 32);
+    const float4* tw4 = reinterpret_cast<const float4*>(twl);
+
+    __shared__ int s_item[2];   // the item rank 0 fetched, by item parity
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) unsigned long long s_bar;   // the column buffer's bytes of one tile
+    cg::cluster_group cluster = cg::this_cluster();
+    const int r = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int a = lane >> 1, h = lane & 1;
+    float4* stage = scr_all + (size_t)warp * FT;   // the warp's scratch: two lines, or the blocks it sends
+    float4* scr = stage + h * (FT / 2);
+    const uint32_t bar = smem_addr(&s_bar);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(&s_tmem)),
+                     "r"(S::TM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < 16 * 32; i += S::THR) twl[i] = twg[((i & 31) * (i >> 5)) & (FT - 1)];
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const uint32_t tm_taper = tmem + (uint32_t)((warp >> 2) * S::TM_TAPER);
+    const uint32_t tm_park = tmem + (uint32_t)(S::TM_PARK0 + (warp >> 2) * S::TM_PARK);
+    const uint32_t tm_acc = tmem + (uint32_t)(S::TM_ACC0 + (warp >> 2) * S::TM_ACC);
+#pragma unroll 1
+    for (int q = 0; q < 2 * S::ROUNDS; ++q) {   // round q / 2, row q % 2 of this half's pair
+        const float* ta =
+            taper + (size_t)(r * S::R + 4 * (warp + q / 2 * S::NW) + 2 * h + (q & 1)) * FT + 2 * a;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float2 w = __ldg(reinterpret_cast<const float2*>(ta + 32 * j));
+            v[2 * j] = w.x;
+            v[2 * j + 1] = w.y;
+        }
+        tmem_put32(tm_taper + 32 * q, v);
+    }
+
+    int ipar = 0;       // s_item parity
+    uint32_t phase = 0; // of s_bar: one per tile
+    bool dead = false;  // a wait gave up: no further waits (the results are void, err is set)
+    for (;;) {
+        // as in k_fused_spectrum: items in order from one counter, each slot
+        // rewritten two items later
+        if (r == 0 && tid == 0) s_item[ipar] = take_front(next_item, nitems);
+        cluster.sync();
+        const int it = *cluster.map_shared_rank(&s_item[ipar], 0);
+        ipar ^= 1;
+        if (it >= nitems) break;
+        const int4 item = items[it];   // (image, first tile, end tile, item index)
+        const FusedTab im = imgs[item.x];
+        const bool v2 = im.vec == 2;
+        // this lane's first two samples of its half's first row pair in tile t
+        auto rows_of = [&](int t) {
+            return im.img +
+                   (size_t)(im.offy + t / im.ntx * im.stride + r * S::R + 4 * warp + 2 * h) * im.pitch + im.offx +
+                   t % im.ntx * im.stride + 2 * a;
+        };
+        // tile mean = four block sums / tile area
+        auto mean_of = [&](int t) {
+            const double* bs = im.bsum + (size_t)(t / im.ntx) * im.nbx + t % im.ntx;
+            return (float)((bs[0] + bs[1] + bs[im.nbx] + bs[im.nbx + 1]) / ((double)FT * FT));
+        };
+        for (int i = tid; i < FT; i += S::THR) accN[i] = 0.0f;
+        // rows in flight: na, nb hold a row pair of this half, quarter by quarter
+        float2 na[16], nb[16];
+        auto load_part = [&](const float* p, int part) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                na[4 * part + j] = row2(p + 32 * (4 * part + j), v2);
+                nb[4 * part + j] = row2(p + im.pitch + 32 * (4 * part + j), v2);
+            }
+        };
+        auto load_rows = [&](const float* p) {
+#pragma unroll
+            for (int part = 0; part < 4; ++part) load_part(p, part);
+        };
+        auto park_rows = [&] {
+            float w[32];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                w[2 * j] = na[j].x;
+                w[2 * j + 1] = na[j].y;
+            }
+            tmem_put32(tm_park, w);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                w[2 * j] = nb[j].x;
+                w[2 * j + 1] = nb[j].y;
+            }
+            tmem_put32(tm_park + 32, w);
+        };
+        const size_t half_rows = (size_t)(4 * S::NW) * im.pitch;
+        // the copies out of this warp's staging have been read
+        auto sent = [&] {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+        };
+        const float* src = rows_of(item.y);
+        float mean = mean_of(item.y);
+        load_rows(src);
+        park_rows();
+        load_rows(src + half_rows);
+
+        for (int t = item.y; t < item.z; ++t) {
+            if (tid == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"((uint32_t)S::BUF)
+                             : "memory");
+            const int t1 = t + 1 < item.z ? t + 1 : t;
+            const float* src1 = rows_of(t1);
+            const float mean1 = mean_of(t1);
+
+            // ---- row transforms: four rows per warp and round ------------------
+#pragma unroll
+            for (int q = 0; q < S::ROUNDS; ++q) {
+                float2 e[16], o[16];
+                float w[32];
+                if (q == 0) {
+                    float x[32];
+                    tmem_get32(tm_park, x);
+                    tmem_get32(tm_taper, w);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        e[j].x = (x[2 * j] - mean) * w[2 * j];
+                        o[j].x = (x[2 * j + 1] - mean) * w[2 * j + 1];
+                    }
+                    tmem_get32(tm_park + 32, x);
+                    tmem_get32(tm_taper + 32, w);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        e[j].y = (x[2 * j] - mean) * w[2 * j];
+                        o[j].y = (x[2 * j + 1] - mean) * w[2 * j + 1];
+                    }
+                    fft512_pair(e, o, scr, tw4, lane, [](int) {});
+                } else {
+                    tmem_get32(tm_taper + 64, w);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        e[j].x = (na[j].x - mean) * w[2 * j];
+                        o[j].x = (na[j].y - mean) * w[2 * j + 1];
+                    }
+                    tmem_get32(tm_taper + 96, w);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        e[j].y = (nb[j].x - mean) * w[2 * j];
+                        o[j].y = (nb[j].y - mean) * w[2 * j + 1];
+                    }
+                    sent();
+                    fft512_pair(e, o, scr, tw4, lane, [&](int part) { load_part(src1, part); });
+                }
+                __syncwarp();
+                // Z[K] and Z[512 - K], K < 256, to CTA K / C: the block's halves
+                // hold [column][h] of each, column K % C at K ^ 2 (row block & 3):
+                // neither these stores nor the column loads have bank conflicts.
+                // (Z[0] and Z[256] meet in column 0.)
+                float2* zk = reinterpret_cast<float2*>(stage) + ((a ^ (2 * (warp & 3))) * 2 + h);
+                float2* zn = reinterpret_cast<float2*>(stage) + S::BLOCK / 2 + ((((16 - a) & 15) ^ (2 * (warp & 3))) * 2 + h);
+                const int up = a == 0 ? 1 : 0;   // bin 256 + 16 k is column 256 - 16 k: one group of 16 up
+#pragma unroll
+                for (int kk = 0; kk < 16; ++kk) {
+                    zk[(kk >> 1) * S::BLOCK + (kk & 1) * 32] = e[P16(kk)];
+                    const int g = (15 - kk + up) & 15;   // column group of bin a + 16 kk + 256
+                    zn[(g >> 1) * S::BLOCK + (g & 1) * 32] = o[P16(kk)];
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (q == 0 && t > item.y) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+                if (lane < S::CL) {
+                    const uint32_t block = smem_addr(colbuf + (size_t)(S::R / 4 * r + warp + q * S::NW) * S::BLOCK);
+                    asm volatile(
+                        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                        ::"r"(cluster_addr(block, lane)),
+                        "r"(smem_addr(stage + lane * (S::BLOCK / 2))), "r"((uint32_t)(S::BLOCK * sizeof(float2))),
+                        "r"(cluster_addr(bar, lane))
+                        : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            }
+            sent();
+            // every block of this tile has landed in the column buffer
+            if (!dead && !wait_phase(bar, phase)) {
+                dead = true;
+                if (err) atomicExch(err, 8);
+            }
+            phase ^= 1;
+
+            // ---- column transforms: two columns per warp and round --------------
+#pragma unroll
+            for (int q = 0; q < S::ROUNDS; ++q) {
+                const int cl = 2 * (warp + q * S::NW) + h;   // local column
+                float2 e[16], o[16];
+                // rows 32 j + 2a, + 1 (block 8 j + a / 2): the two real rows' bins
+                // from one FFT's, twice their value (the 1/2 of the split is applied
+                // once, exactly, to the averaged spectrum in k_item_reduce)
+                const float2* col = colbuf + (a >> 1) * S::BLOCK + (cl ^ (a & 6)) * 2 + (a & 1);
+                const bool packed = q == 0 && r == 0 && warp == 0;   // column 0 on the even lanes: (0, 256)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float2 zk = col[8 * j * S::BLOCK], zn = col[8 * j * S::BLOCK + S::BLOCK / 2];
+                    e[j] = make_float2(zk.x + zn.x, zk.y - zn.y);
+                    o[j] = make_float2(zk.y + zn.y, zn.x - zk.x);
+                    if (packed && h == 0) {
+                        e[j] = make_float2(2.0f * zk.x, 2.0f * zn.x);
+                        o[j] = make_float2(2.0f * zk.y, 2.0f * zn.y);
+                    }
+                }
+                if (q == 0) {
+                    park_rows();
+                    fft512_pair(e, o, scr, tw4, lane, [&](int part) { load_part(src1 + half_rows, part); });
+                } else {
+                    fft512_pair(e, o, scr, tw4, lane, [](int) {});
+                }
+                // this warp's column loads of the tile are done
+                if (q == S::ROUNDS - 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+                float acc[32];
+                if (t > item.y) {
+                    tmem_get32(tm_acc + 32 * q, acc);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) acc[k] = 0.0f;
+                }
+                if (packed) {
+                    packed_column(e, o, lane, accN, acc);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        acc[k] += amp_xy(e[P16(k)].x, e[P16(k)].y);
+                        acc[k + 16] += amp_xy(o[P16(k)].x, o[P16(k)].y);
+                    }
+                }
+                tmem_put32(tm_acc + 32 * q, acc);
+            }
+            src = src1;
+            mean = mean1;
+        }
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // of the last tile's arrive
+        // ---- write this item's partial spectrum (DC moved to row 256) -----------
+        float* out = partial + (size_t)item.w * FCX * FT;
+#pragma unroll
+        for (int q = 0; q < S::ROUNDS; ++q) {
+            const int kx = S::C * r + 2 * (warp + q * S::NW) + h;
+            float acc[32];
+            tmem_get32(tm_acc + 32 * q, acc);
+            if (q == 0 && r == 0 && warp == 0) mirror_column(lane, acc);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+                const int yd = (a + 16 * k + FT / 2) & (FT - 1);
+                out[(size_t)yd * FCX + kx] = acc[k];
+            }
+        }
+        __syncthreads();
+        if (r == 0)
+            for (int ky = tid; ky < FT; ky += S::THR)
+                out[(size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] = accN[ky <= FT / 2 ? ky : FT - ky];
+        __syncthreads();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster.sync();   // keep shared memory alive until every peer is done
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "r"(S::TM_COLS)
+                     : "memory");
+}
+
 // ---- tiles on the SMs that the clusters leave free --------------------------
 // 8-CTA clusters fit twice per GPC, so some SMs stay idle beside the cluster
 // kernel.  One CTA of this kernel runs on each of them, takes work items
 // from the same counter and transforms whole tiles alone: the row spectra go
 // to the CTA's column buffer in global memory (L2-resident scratch), the
 // column transforms read them back, and the item's |F| sums live in a second
-// global buffer ([column][row]) until the item ends, when they are written
-// to the item's partial spectrum in the cluster kernel's layout.  The
-// transforms, the split and the order of every addition are those of
-// k_fused_spectrum, so an item's partial spectrum does not depend on which
-// kernel took it.
+// global buffer until the item ends, when they are written to the item's
+// partial spectrum in the cluster kernel's layout.  The transforms, the split
+// and the order of every addition are those of the cluster kernels, so an
+// item's partial spectrum does not depend on which kernel took it.  Two lines
+// per warp (fft512_pair), the next round's rows and taper, or columns, in
+// flight during each transform.
 constexpr int kSoloThreads = 256;
 constexpr int kSoloWarps = kSoloThreads / 32;
 constexpr int kSoloYS = FT + 2;                                      // column stride, float2
 constexpr size_t kSoloColFloat2 = (size_t)(FT / 2) * kSoloYS;        // columns 0..255 of one tile
-constexpr size_t kSoloAccFloats = (size_t)(FT / 2) * FT;             // |F| sums, [column][row]
-constexpr size_t kSoloSmem = (size_t)kSoloWarps * FSCR * sizeof(float2) + 16 * 32 * sizeof(float2) +
+constexpr size_t kSoloAccFloats = (size_t)(FT / 2) * FT;             // |F| sums, [column pair][8][lane][4]
+constexpr size_t kSoloSmem = (size_t)kSoloWarps * 2 * FT * sizeof(float2) + 16 * 32 * sizeof(float2) +
                              FT * sizeof(float);
+constexpr int kSoloRounds = FT / 4 / kSoloWarps;                     // rounds of two row pairs, or two columns, per warp
 
 __global__ void __launch_bounds__(kSoloThreads, 1)
 k_fused_spectrum_solo(const FusedTab* __restrict__ imgs, const int4* __restrict__ items, int nitems,
@@ -515,15 +1072,16 @@ k_fused_spectrum_solo(const FusedTab* __restrict__ imgs, const int4* __restrict_
                       float2* __restrict__ colg_all, float* __restrict__ accg_all)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    float2* scr_all = reinterpret_cast<float2*>(smem);
-    float2* twl = scr_all + kSoloWarps * FSCR;
+    float4* scr_all = reinterpret_cast<float4*>(smem);
+    float2* twl = reinterpret_cast<float2*>(scr_all + kSoloWarps * FT);
+    const float4* tw4 = reinterpret_cast<const float4*>(twl);
     float* accN = reinterpret_cast<float*>(twl + 16 * 32);
     __shared__ int s_item;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m = lane >> 1, p = lane & 1;
-    float2* scr = scr_all + warp * FSCR;
+    const int a = lane >> 1, h = lane & 1;
+    float4* scr = scr_all + (size_t)warp * FT + h * (FT / 2);
     float2* colg = colg_all + (size_t)blockIdx.x * kSoloColFloat2;
-    float* accg = accg_all + (size_t)blockIdx.x * kSoloAccFloats;
+    float4* accg = reinterpret_cast<float4*>(accg_all + (size_t)blockIdx.x * kSoloAccFloats) + lane;
     for (int i = tid; i < 16 * 32; i += kSoloThreads) twl[i] = twg[((i & 31) * (i >> 5)) & (FT - 1)];
     for (;;) {
         __syncthreads();   // the previous item is written; every thread has read s_item
@@ -533,110 +1091,121 @@ k_fused_spectrum_solo(const FusedTab* __restrict__ imgs, const int4* __restrict_
         if (it >= nitems) break;
         const int4 item = items[it];   // (image, first tile, end tile, item index)
         const FusedTab im = imgs[item.x];
+        const bool v2 = im.vec == 2;
         for (int i = tid; i < FT; i += kSoloThreads) accN[i] = 0.0f;   // read after the row phase's barrier
         for (int t = item.y; t < item.z; ++t) {
             const bool first = t == item.y;
             const int tx = t % im.ntx, ty = t / im.ntx;
-            const float* src = im.img + (size_t)(im.offy + ty * im.stride) * im.pitch + im.offx + tx * im.stride;
             const double* bs = im.bsum + (size_t)ty * im.nbx + tx;
             const float mean = (float)((bs[0] + bs[1] + bs[im.nbx] + bs[im.nbx + 1]) / ((double)FT * FT));
+            // this half's row pair of round q: rows 4 (warp + 8 q) + 2h, + 1
+            const int Y = 4 * warp + 2 * h;
+            const float* src =
+                im.img + (size_t)(im.offy + ty * im.stride + Y) * im.pitch + im.offx + tx * im.stride + 2 * a;
+            const float* tap = taper + (size_t)Y * FT + 2 * a;
 
-            // ---- row transforms: 256 row pairs, the next pair prefetched --------
-            float na[16], nb[16];
+            // ---- row transforms: the next round's rows and taper in flight ------
             {
-                const float* ga = src + (size_t)(2 * warp) * im.pitch;
+                float2 na[16], nb[16], wa[16], wb[16];
+                auto load_part = [&](int q, int part) {
+                    const float* p = src + (size_t)(4 * kSoloWarps * q) * im.pitch;
+                    const float* w = tap + (size_t)(4 * kSoloWarps * q) * FT;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    na[j] = __ldg(ga + 32 * j + lane);
-                    nb[j] = __ldg(ga + im.pitch + 32 * j + lane);
-                }
-            }
-            for (int q = 0; q < FT / 2 / kSoloWarps; ++q) {
-                const int Y0 = 2 * (warp + kSoloWarps * q);
-                float ca[16], cb[16];
+                    for (int j = 4 * part; j < 4 * part + 4; ++j) {
+                        na[j] = row2(p + 32 * j, v2);
+                        nb[j] = row2(p + im.pitch + 32 * j, v2);
+                        wa[j] = __ldg(reinterpret_cast<const float2*>(w + 32 * j));
+                        wb[j] = __ldg(reinterpret_cast<const float2*>(w + FT + 32 * j));
+                    }
+                };
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    ca[j] = na[j];
-                    cb[j] = nb[j];
-                }
-                if (q + 1 < FT / 2 / kSoloWarps) {
-                    const float* ga = src + (size_t)(Y0 + 2 * kSoloWarps) * im.pitch;
+                for (int part = 0; part < 4; ++part) load_part(0, part);
+#pragma unroll 1
+                for (int q = 0; q < kSoloRounds; ++q) {
+                    float2 e[16], o[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        na[j] = __ldg(ga + 32 * j + lane);
-                        nb[j] = __ldg(ga + im.pitch + 32 * j + lane);
+                        e[j] = make_float2((na[j].x - mean) * wa[j].x, (nb[j].x - mean) * wb[j].x);
+                        o[j] = make_float2((na[j].y - mean) * wa[j].y, (nb[j].y - mean) * wb[j].y);
                     }
+                    const int qn = min(q + 1, kSoloRounds - 1);
+                    fft512_pair(e, o, scr, tw4, lane, [&](int part) { load_part(qn, part); });
+                    float2* dst = colg + (size_t)a * kSoloYS + Y + 4 * kSoloWarps * q;
+                    split_rows(e, o, lane, [&](int kk, float4 AB) {
+                        *reinterpret_cast<float4*>(dst + (size_t)(16 * kk) * kSoloYS) = AB;
+                    });
                 }
-                float2 v[16];
-                const float* ta = taper + (size_t)Y0 * FT;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    int X = 32 * j + lane;
-                    v[j] = make_float2((ca[j] - mean) * __ldg(ta + X), (cb[j] - mean) * __ldg(ta + FT + X));
-                }
-                fft512_warp(v, scr, twl, lane);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) scr[sslot(m + 16 * k + 256 * p)] = v[P16(k)];
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int K = lane + 32 * i;
-                    float2 zk = scr[sslot(K)], zn = scr[sslot((FT - K) & (FT - 1))];
-                    float4 AB = make_float4(zk.x + zn.x, zk.y - zn.y, zk.y + zn.y, zn.x - zk.x);
-                    if (K == 0) {
-                        float2 zh = scr[sslot(FT / 2)];
-                        AB = make_float4(2.0f * zk.x, 2.0f * zh.x, 2.0f * zk.y, 2.0f * zh.y);
-                    }
-                    *reinterpret_cast<float4*>(colg + (size_t)K * kSoloYS + Y0) = AB;
-                }
-                __syncwarp();
             }
             __syncthreads();   // the tile's column buffer is complete
 
             // ---- column transforms from the global column buffer ----------------
-            for (int cc = 0; cc < FT / 2 / kSoloWarps; ++cc) {
-                const int K = warp + kSoloWarps * cc;   // 0 = packed (0, 256)
-                float2 v[16];
-                const float2* col = colg + (size_t)K * kSoloYS;
+            {
+                const float2* col = colg + (size_t)(2 * warp + h) * kSoloYS + 2 * a;   // column 2 (warp + 8 q) + h
+                float4 nx[16];
+                auto load_part = [&](int q, int part) {
+                    const float2* p = col + (size_t)(2 * kSoloWarps * q) * kSoloYS;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = col[32 * j + lane];
-                float* a = accg + (size_t)K * FT;
-                float av[16];
+                    for (int j = 4 * part; j < 4 * part + 4; ++j) nx[j] = *reinterpret_cast<const float4*>(p + 32 * j);
+                };
 #pragma unroll
-                for (int k = 0; k < 16; ++k) av[k] = first ? 0.0f : a[m + 16 * k + 256 * p];
-                fft512_warp(v, scr, twl, lane);
-                if (K != 0) {
+                for (int part = 0; part < 4; ++part) load_part(0, part);
+#pragma unroll 1
+                for (int q = 0; q < kSoloRounds; ++q) {
+                    float2 e[16], o[16];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        float2 z = v[P16(k)];
-                        a[m + 16 * k + 256 * p] = av[k] + amp(z.x, z.y);
+                    for (int j = 0; j < 16; ++j) {
+                        e[j] = make_float2(nx[j].x, nx[j].y);
+                        o[j] = make_float2(nx[j].z, nx[j].w);
                     }
-                } else {
+                    float4* ap = accg + (size_t)(warp + kSoloWarps * q) * 8 * 32;
+                    float acc[32];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) scr[sslot(m + 16 * k + 256 * p)] = v[P16(k)];
-                    __syncwarp();
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        int Kk = m + 16 * k + 256 * p;
-                        float2 zk = v[P16(k)], zn = scr[sslot((FT - Kk) & (FT - 1))];
-                        float ax = 0.5f * (zk.x + zn.x), ay = 0.5f * (zk.y - zn.y);
-                        float bx = 0.5f * (zk.y + zn.y), by = -0.5f * (zk.x - zn.x);
-                        a[Kk] = av[k] + amp(ax, ay);
-                        accN[Kk] += amp(bx, by);
+                    for (int i = 0; i < 8; ++i) {
+                        const float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ap[32 * i];
+                        acc[4 * i] = v.x;
+                        acc[4 * i + 1] = v.y;
+                        acc[4 * i + 2] = v.z;
+                        acc[4 * i + 3] = v.w;
                     }
-                    __syncwarp();
+                    const int qn = min(q + 1, kSoloRounds - 1);
+                    fft512_pair(e, o, scr, tw4, lane, [&](int part) { load_part(qn, part); });
+                    if (q == 0 && warp == 0) {   // column 0 is the packed (0, 256)
+                        packed_column(e, o, lane, accN, acc);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) {
+                            acc[k] += amp_xy(e[P16(k)].x, e[P16(k)].y);
+                            acc[k + 16] += amp_xy(o[P16(k)].x, o[P16(k)].y);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        ap[32 * i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
                 }
             }
-            __syncthreads();   // the column buffer is free again; the sums are complete
+            __syncthreads();   // the column buffer is free again; accN is complete
         }
         // ---- the item's partial spectrum (DC moved to row 256) ------------------
         float* out = partial + (size_t)item.w * FCX * FT;
-        for (int i = tid; i < (FT / 2) * FT; i += kSoloThreads) {
-            const int kx = i / FT, ky = i - kx * FT;
-            out[(size_t)((ky + FT / 2) & (FT - 1)) * FCX + kx] = accg[i];
+#pragma unroll 1
+        for (int q = 0; q < kSoloRounds; ++q) {
+            const float4* ap = accg + (size_t)(warp + kSoloWarps * q) * 8 * 32;
+            float acc[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 v = ap[32 * i];
+                acc[4 * i] = v.x;
+                acc[4 * i + 1] = v.y;
+                acc[4 * i + 2] = v.z;
+                acc[4 * i + 3] = v.w;
+            }
+            if (q == 0 && warp == 0) mirror_column(lane, acc);
+            const int kx = 2 * (warp + kSoloWarps * q) + h;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) out[(size_t)((a + 16 * k + FT / 2) & (FT - 1)) * FCX + kx] = acc[k];
         }
         for (int ky = tid; ky < FT; ky += kSoloThreads)
-            out[(size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] = accN[ky];
+            out[(size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] = accN[ky <= FT / 2 ? ky : FT - ky];
     }
 }
 
@@ -701,6 +1270,57 @@ cudaError_t prepare_kernel()
     if (e != cudaSuccess) return e;
     if (S::CL > 8) e = cudaFuncSetAttribute(k_fused_spectrum<S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
+}
+
+template <class S>
+cudaLaunchConfig_t pair_cfg(int nclusters, cudaStream_t st, cudaLaunchAttribute* attr)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nclusters * S::CL, 1, 1);
+    cfg.blockDim = dim3(S::THR, 1, 1);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S::CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <class S>
+cudaError_t prepare_pair()
+{
+    cudaError_t e = init_constants();
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_fused_spectrum_pair<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e == cudaSuccess && S::CL > 8)
+        e = cudaFuncSetAttribute(k_fused_spectrum_pair<S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+template <class S>
+cudaError_t max_pair_clusters(int* n)
+{
+    *n = 0;
+    cudaError_t e = prepare_pair<S>();
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = pair_cfg<S>(64, nullptr, attr);
+    return cudaOccupancyMaxActiveClusters(n, (void*)k_fused_spectrum_pair<S>, &cfg);
+}
+
+template <class S>
+cudaError_t launch_pair(int nclusters, cudaStream_t st, const void* descs, const int4* items, int nitems,
+                        const float* taper, const float2* tw, float* partial, unsigned long long* next_item, int* err)
+{
+    cudaError_t e = prepare_pair<S>();
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = pair_cfg<S>(nclusters, st, attr);
+    return cudaLaunchKernelEx(&cfg, k_fused_spectrum_pair<S>, reinterpret_cast<const FusedTab*>(descs), items, nitems,
+                              taper, tw, partial, next_item, err);
 }
 
 template <class S>
@@ -891,35 +1511,27 @@ cudaError_t launch_lowpass512(const float* ctf0, const float2* tw, double bfacto
     return cudaGetLastError();
 }
 
-// Picks the cluster shape that covers the most SMs: 16-CTA clusters (double
-// buffered) when the device can co-schedule them, else 8-CTA clusters.
+// Picks the cluster shape: 8-CTA clusters with two lines per warp wherever they
+// can be resident (16 micrographs of 4096 x 4096: 2.30 ms; the one-line shapes
+// 816, 168, 162 and 16 take 3.53, 3.51, 3.84 and 4.81 ms), else 16-CTA ones.
 cudaError_t fused_max_clusters(int* n, int* shape)
 {
-    int n16 = 0, n8 = 0;
-    if (max_clusters<Shape16>(&n16) != cudaSuccess) {
-        cudaGetLastError();
-        n16 = 0;
-    }
-    cudaError_t e = max_clusters<Shape8>(&n8);
-    if (e != cudaSuccess && n16 == 0) return e;
-    if (n16 * 16 >= n8 * 8 && n16 > 0) {
-        *n = n16;
-        *shape = 16;
-    } else {
-        *n = n8;
-        *shape = 8;
-    }
-    return cudaSuccess;
+    cudaError_t e = max_pair_clusters<Pair8>(n);
+    *shape = 8;
+    if (e == cudaSuccess && *n > 0) return e;
+    cudaGetLastError();
+    *shape = 16;
+    return max_clusters<Shape16>(n);
 }
 
-// Co-resident clusters of one shape: 8 (8 CTAs x 8 warps), 816 (8 CTAs x 16
+// Co-resident clusters of one shape: 8 (8 CTAs x 8 warps, two lines per warp), 816 (8 CTAs x 16
 // warps, 128 registers), 16 (16 CTAs x 16 warps, double buffered), 162 (16
 // CTAs x 8 warps, two CTAs per SM), 168 (16 CTAs x 8 warps, double buffered).
 cudaError_t fused_clusters_of(int shape, int* n)
 {
     *n = 0;
     switch (shape) {
-    case 8: return max_clusters<Shape8>(n);
+    case 8: return max_pair_clusters<Pair8>(n);
     case 816: return max_clusters<Shape8W16>(n);
     case 16: return max_clusters<Shape16>(n);
     case 162: return max_clusters<Shape16x2>(n);
@@ -935,8 +1547,8 @@ size_t solo_scratch_floats(int nsolo) { return (size_t)nsolo * kSoloAccFloats; }
 cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blocks, const int4* items,
                          int nitems, const int* first, const float* inv, int img0, int nimg,
                          const float* taper, const float2* tw, float* partial, float* raw,
-                         unsigned long long* next_item, int nclusters, int shape, cudaStream_t st, cudaEvent_t ev0,
-                         cudaEvent_t ev1, const SoloLaunch* solo)
+                         unsigned long long* next_item, int* err, int nclusters, int shape, cudaStream_t st,
+                         cudaEvent_t ev0, cudaEvent_t ev1, const SoloLaunch* solo)
 {
     if (nclusters < 1) nclusters = 1;
     k_block_sums<<<dim3(max_blocks, nimg), 256, 0, st>>>(reinterpret_cast<const FusedTab*>(descs) + img0,
@@ -972,15 +1584,15 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
         e = cudaLaunchKernelEx(&cfg, k_fused_spectrum<Shape8W16>, reinterpret_cast<const FusedTab*>(descs),
                                items, nitems, taper, tw, partial, next_item);
     } else {
-        if ((e = prepare_kernel<Shape8>()) != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg = fused_cfg<Shape8>(nclusters, st, attr);
-        e = cudaLaunchKernelEx(&cfg, k_fused_spectrum<Shape8>, reinterpret_cast<const FusedTab*>(descs), items,
-                               nitems, taper, tw, partial, next_item);
+        e = launch_pair<Pair8>(nclusters, st, descs, items, nitems, taper, tw, partial, next_item, err);
     }
     if (e != cudaSuccess) return e;
     if (use_solo) {
         // after the cluster launch, so that its clusters are placed first and
         // these CTAs land on the SMs they leave free
+        if ((e = cudaFuncSetAttribute(k_fused_spectrum_solo, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSoloSmem)) != cudaSuccess)
+            return e;
         k_fused_spectrum_solo<<<solo->n, kSoloThreads, kSoloSmem, solo->st>>>(
             reinterpret_cast<const FusedTab*>(descs), items, nitems, taper, tw, partial, next_item,
             solo->reserve_per_cluster * nclusters, solo->col, solo->acc);
@@ -1025,6 +1637,7 @@ struct NaMeta {
     int first[2];
     float inv[1];
     unsigned long long next_item;
+    int err;   // a bounded wait of the tile kernel gave up
 };
 constexpr size_t kNaBytes = kNaMetaOff + ((sizeof(NaMeta) + 255) / 256) * 256;
 
@@ -1154,7 +1767,7 @@ extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, 
                                  nitems, dmeta->first, dmeta->inv, 0, 1,
                                  reinterpret_cast<const float*>(base + kNaTaperOff),
                                  reinterpret_cast<const float2*>(base + kNaTwOff),
-                                 reinterpret_cast<float*>(base), dev_raw_out, &dmeta->next_item, ncl,
+                                 reinterpret_cast<float*>(base), dev_raw_out, &dmeta->next_item, &dmeta->err, ncl,
                                  g_na_shape[dev], st, nullptr, nullptr);
     if (e != cudaSuccess) return GCF_ERR_CUDA;
     return GCF_OK;
