@@ -246,7 +246,7 @@ struct gcf_ctx {
     DBuf<float2> tw512;
     DBuf<FusedImageDesc> f_desc;
     DBuf<int4> f_items;
-    DBuf<int> f_first;
+    DBuf<int> f_first, f_group;
     DBuf<float> f_inv, f_partial;
     DBuf<unsigned long long> f_next;   // item queues of the tile kernel launches
     // cluster-less tile CTAs beside each cluster launch (SMs the clusters
@@ -762,7 +762,24 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
     first.assign(nm + 1, 0);
     ctx->f_blocks_h.assign(nm, 0);
     std::vector<float> inv(nm);
+    std::vector<int> group(nm, 1);
     std::vector<size_t> boff(nm);
+    // Too few items for the clusters: the tiles themselves are handed out, and
+    // k_item_reduce adds each item's tiles in order, as its cluster would have
+    // (the same bits).  A tile handed out alone costs 18 us of a cluster
+    // instead of 11.8 (its rows are not read ahead, its sums are written) and
+    // 0.25 us in the reduction, so it pays while the plan's tiles are fewer
+    // than 8 times the longest item's: a 1024 x 1024 frame (9 tiles, 1 item)
+    // 106 -> 26 us, 2048 x 2048 (49, 3) 200 -> 82 us, 3838 x 3710 (169, 8)
+    // 260 -> 246 us; but 4096 x 4096 (225, 10) 271 -> 316 us.
+    int tiles = 0, longest = 0;
+    for (const MicImage& m : mics) {
+        const Layout L = tile_layout(m.w, m.h, T);
+        const int nt = std::max(L.ntx, 0) * std::max(L.nty, 0), nch = (nt + kItemTiles - 1) / kItemTiles;
+        tiles += nt;
+        if (nch > 0) longest = std::max(longest, (nt + nch - 1) / nch);
+    }
+    const bool single = tiles < 8 * longest;
     size_t nblk = 0;
     for (int i = 0; i < nm; ++i) {
         const MicImage& m = mics[i];
@@ -787,8 +804,10 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
         first[i] = (int)items.size();
         int nch = (nt + kItemTiles - 1) / kItemTiles;
         int chunk = (nt + nch - 1) / nch;
-        for (int t0 = 0; t0 < nt; t0 += chunk)
-            items.push_back(make_int4(i, t0, std::min(nt, t0 + chunk), (int)items.size()));
+        group[i] = single ? chunk : 1;
+        const int step = single ? 1 : chunk;
+        for (int t0 = 0; t0 < nt; t0 += step)
+            items.push_back(make_int4(i, t0, std::min(nt, t0 + step), (int)items.size()));
     }
     first[nm] = (int)items.size();
     int ni = (int)items.size();
@@ -803,12 +822,14 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
     CK(ctx->f_desc.ensure(nm));
     CK(ctx->f_items.ensure(ni));
     CK(ctx->f_first.ensure(nm + 1));
+    CK(ctx->f_group.ensure(nm));
     CK(ctx->f_inv.ensure(nm));
     CK(ctx->f_partial.ensure((size_t)ni * cx * T));
     CK(ctx->f_next.ensure(nm));
     CK(h2d(ctx, ctx->f_desc.p, d.data(), nm * sizeof(FusedImageDesc), ctx->st));
     CK(h2d(ctx, ctx->f_items.p, items.data(), ni * sizeof(int4), ctx->st));
     CK(h2d(ctx, ctx->f_first.p, first.data(), (nm + 1) * sizeof(int), ctx->st));
+    CK(h2d(ctx, ctx->f_group.p, group.data(), nm * sizeof(int), ctx->st));
     CK(h2d(ctx, ctx->f_inv.p, inv.data(), nm * sizeof(float), ctx->st));
     return GCF_OK;
 }
@@ -871,7 +892,7 @@ gcf_status fused_launch(gcf_ctx* ctx, int m0, int m1, float* raw_out, cudaStream
     SoloLaunch sl{};
     if (solo) CKS(solo_setup(ctx, &sl));
     CK(launch_fused(ctx->f_desc.p, ctx->f_bsum_ptr.p, max_blocks, ctx->f_items.p + first[m0], ni, ctx->f_first.p,
-                    ctx->f_inv.p, m0, m1 - m0, ctx->taper.p, ctx->tw512.p, ctx->f_partial.p, raw_out,
+                    ctx->f_group.p, ctx->f_inv.p, m0, m1 - m0, ctx->taper.p, ctx->tw512.p, ctx->f_partial.p, raw_out,
                     ctx->f_next.p + m0, ctx->dev_err.p, ncl, ctx->fused_shape, st, e0, e1, solo ? &sl : nullptr));
     ctx->launches += (solo && sl.n > 0 && ni > ncl) ? 4 : 3;
     return GCF_OK;
@@ -1980,6 +2001,7 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->f_desc.release();
     ctx->f_items.release();
     ctx->f_first.release();
+    ctx->f_group.release();
     ctx->f_inv.release();
     ctx->f_partial.release();
     ctx->f_next.release();

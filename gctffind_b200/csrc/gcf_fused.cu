@@ -33,6 +33,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -698,6 +699,7 @@ struct PairShape {
     static constexpr int TM_COLS = 512 / MINB;
     static_assert(ROUNDS == 2 && R == 4 * NW * ROUNDS && NW % 4 == 0 && CL <= 16, "shape");
     static_assert(TM_PARK0 + NW / 4 * TM_PARK <= TM_COLS, "tensor memory");
+    static_assert(C == 32 && BUF >= (size_t)FT * 33 * sizeof(float), "write-out stage");
 };
 using Pair8 = PairShape<8, 8>;
 
@@ -1017,23 +1019,27 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
         }
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // of the last tile's arrive
         // ---- write this item's partial spectrum (DC moved to row 256) -----------
-        float* out = partial + (size_t)item.w * FCX * FT;
+        // through the column buffer ([row][33], free until the next item's
+        // cluster barrier), so that a warp writes 32 adjacent columns of a row
+        float* stage_out = reinterpret_cast<float*>(smem);
+        __syncthreads();   // every warp is done with the column buffer
 #pragma unroll
         for (int q = 0; q < S::ROUNDS; ++q) {
-            const int kx = S::C * r + 2 * (warp + q * S::NW) + h;
             float acc[32];
             tmem_get32(tm_acc + 32 * q, acc);
             if (q == 0 && r == 0 && warp == 0) mirror_column(lane, acc);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                const int yd = (a + 16 * k + FT / 2) & (FT - 1);
-                out[(size_t)yd * FCX + kx] = acc[k];
-            }
+            for (int k = 0; k < 32; ++k)
+                stage_out[((a + 16 * k + FT / 2) & (FT - 1)) * 33 + 2 * (warp + q * S::NW) + h] = acc[k];
         }
         __syncthreads();
+        float* out = partial + (size_t)item.w * FCX * FT + S::C * r + lane;
+#pragma unroll 8
+        for (int y = warp; y < FT; y += S::NW) out[(size_t)y * FCX] = stage_out[y * 33 + lane];
         if (r == 0)
             for (int ky = tid; ky < FT; ky += S::THR)
-                out[(size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] = accN[ky <= FT / 2 ? ky : FT - ky];
+                partial[(size_t)item.w * FCX * FT + (size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] =
+                    accN[ky <= FT / 2 ? ky : FT - ky];
         __syncthreads();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1210,15 +1216,30 @@ k_fused_spectrum_solo(const FusedTab* __restrict__ imgs, const int4* __restrict_
 }
 
 // raw[img] = sum of the img's item partials (in item order) / ntiles / 2.
+// group[img] > 1: each partial is one tile, and that many consecutive ones make
+// an item; their FP32 sum, in tile order, is what a cluster that takes the
+// whole item accumulates, bit for bit.
 __global__ void k_item_reduce(const float* __restrict__ partial, const int* __restrict__ first,
-                              const float* __restrict__ inv, float* __restrict__ raw)
+                              const int* __restrict__ group, const float* __restrict__ inv, float* __restrict__ raw)
 {
     const int n = FCX * FT;
     int img = blockIdx.y;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double s = 0.0;
-    for (int k = first[img]; k < first[img + 1]; ++k) s += partial[(size_t)k * n + i];
+    const int end = first[img + 1], g = group ? group[img] : 1;
+    const float* p = partial + i;
+    if (g == 1) {
+        for (int k = first[img]; k < end; ++k) s += p[(size_t)k * n];
+    } else {
+        for (int k = first[img]; k < end; k += g) {
+            float f = 0.0f;
+            const int m = min(g, end - k);
+#pragma unroll 8
+            for (int u = 0; u < m; ++u) f += p[(size_t)(k + u) * n];
+            s += f;
+        }
+    }
     raw[(size_t)img * n + i] = (float)(s * (double)inv[img] * 0.5);   // rows were split without the 1/2
 }
 
@@ -1545,7 +1566,7 @@ size_t solo_scratch_float2(int nsolo) { return (size_t)nsolo * kSoloColFloat2; }
 size_t solo_scratch_floats(int nsolo) { return (size_t)nsolo * kSoloAccFloats; }
 
 cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blocks, const int4* items,
-                         int nitems, const int* first, const float* inv, int img0, int nimg,
+                         int nitems, const int* first, const int* group, const float* inv, int img0, int nimg,
                          const float* taper, const float2* tw, float* partial, float* raw,
                          unsigned long long* next_item, int* err, int nclusters, int shape, cudaStream_t st,
                          cudaEvent_t ev0, cudaEvent_t ev1, const SoloLaunch* solo)
@@ -1602,7 +1623,7 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
     }
     if (ev1 && (e = record_timing(ev1, st)) != cudaSuccess) return e;
     dim3 g((FCX * FT + 255) / 256, nimg);
-    k_item_reduce<<<g, 256, 0, st>>>(partial, first + img0, inv + img0, raw);
+    k_item_reduce<<<g, 256, 0, st>>>(partial, first + img0, group ? group + img0 : nullptr, inv + img0, raw);
     return cudaGetLastError();
 }
 
@@ -1748,7 +1769,9 @@ extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, 
                      ((uintptr_t)dev_img % 8) == 0) ? 2 : 1;
     meta.desc.nbx = ntx + 1;
     meta.bsum_ptr[0] = bsum;
-    int nitems = nt < kNaMaxItems ? nt : kNaMaxItems;
+    // no more items than clusters where that many fit: 294 tiles (5760 x 4092)
+    // as 16 items on 15 clusters took two rounds, 355 us against 237 us
+    int nitems = std::min(nt, std::min(kNaMaxItems, std::max(clusters, 1)));
     int chunk = (nt + nitems - 1) / nitems;
     nitems = 0;
     for (int t0 = 0; t0 < nt; t0 += chunk, ++nitems)
@@ -1764,7 +1787,7 @@ extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, 
     if (cudaGetLastError() != cudaSuccess) return GCF_ERR_CUDA;
     int ncl = clusters < nitems ? clusters : nitems;
     cudaError_t e = launch_fused(&dmeta->desc, dmeta->bsum_ptr, (ntx + 1) * (nty + 1), dmeta->items,
-                                 nitems, dmeta->first, dmeta->inv, 0, 1,
+                                 nitems, dmeta->first, nullptr, dmeta->inv, 0, 1,
                                  reinterpret_cast<const float*>(base + kNaTaperOff),
                                  reinterpret_cast<const float2*>(base + kNaTwOff),
                                  reinterpret_cast<float*>(base), dev_raw_out, &dmeta->next_item, &dmeta->err, ncl,

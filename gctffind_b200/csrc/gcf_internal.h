@@ -238,11 +238,12 @@ size_t solo_scratch_floats(int nsolo);
 // Spectra of images img0 .. img0 + nimg - 1 of descs/bsum_out/first/inv.
 // items: the nitems work items of those images, (image, first tile, end
 // tile, item index into partial); first[img]..first[img+1] are the items of
-// image img; inv[img] = 1 / tiles of img; raw: the spectrum of image img0;
+// image img; group (nullable): items of img that are single tiles of one
+// item (see k_item_reduce), 1 for whole items; inv[img] = 1 / tiles of img; raw: the spectrum of image img0;
 // next_item: the launch's 64-bit item queue counter (zeroed on st).
 // err: device flag, set when a bounded wait gave up (the spectra are void).
 cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blocks, const int4* items,
-                         int nitems, const int* first, const float* inv, int img0, int nimg,
+                         int nitems, const int* first, const int* group, const float* inv, int img0, int nimg,
                          const float* taper, const float2* tw, float* partial, float* raw,
                          unsigned long long* next_item, int* err, int nclusters, int shape, cudaStream_t st,
                          cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, const SoloLaunch* solo = nullptr);

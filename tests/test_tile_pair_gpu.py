@@ -52,3 +52,22 @@ def test_cluster_less_ctas_equal_the_clusters(gpu_lib, w, n):
     ctx.close()
     for r in many:
         assert r.as_dict() == one.as_dict()
+
+
+@pytest.mark.parametrize("w,h", [(512, 512), (1024, 1024), (1500, 2049), (3838, 3710)])
+def test_tiles_handed_out_singly_keep_the_bits(gpu_lib, w, h):
+    """One small frame alone (its tiles handed out one by one) and the same
+    frame in a batch that fills the clusters (whole items): the same result."""
+    import torch
+    from gctffind_b200 import synth
+    G = gpu_lib
+    s = synth.MicrographSpec(width=w, height=h, pixel_size=1.4, df_min=13000.0, df_max=13300.0, dose=3.0, seed=w)
+    img = synth.make_micrograph(s, device="cuda")
+    ctx = G.Context(0, 512, 0)
+    op = G.make_optics()
+    one = ctx.run_batch([img], [1.4], op)[0]
+    n = max(9, 16 * 24 // max(1, ((w - 256) // 256) * ((h - 256) // 256)) + 1)
+    many = ctx.run_batch([img] * n, [1.4] * n, op)
+    ctx.close()
+    for r in many:
+        assert r.as_dict() == one.as_dict()
