@@ -346,7 +346,8 @@ bool rescale_gemm_supported(int w, int h, int nw, int nh);
 RescaleGemmLayout rescale_gemm_layout(int w, int h, int nw, int nh);
 // img (w x h, row pitch `pitch` floats) -> out (nw x nh, dense); err: the
 // products' device flag (0 on entry; set if a bounded wait gave up).
-cudaError_t launch_rescale_gemm(const float* img, long long pitch, int w, int h, int nw, int nh,
+// have_maps: bf already holds the crop maps of these four sizes.
+cudaError_t launch_rescale_gemm(const float* img, long long pitch, int w, int h, int nw, int nh, bool have_maps,
                                 __nv_bfloat16* bf, float* f32, int* err, float* out, cudaStream_t st);
 
 // gcf_contract.cu: the BF16 candidate contraction.

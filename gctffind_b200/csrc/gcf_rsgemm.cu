@@ -264,7 +264,7 @@ RescaleGemmLayout rescale_gemm_layout(int w, int h, int nw, int nh)
     return L;
 }
 
-cudaError_t launch_rescale_gemm(const float* img, long long pitch, int w, int h, int nw, int nh,
+cudaError_t launch_rescale_gemm(const float* img, long long pitch, int w, int h, int nw, int nh, bool have_maps,
                                 __nv_bfloat16* bf, float* f32, int* err, float* out, cudaStream_t st)
 {
     if (!rescale_gemm_supported(w, h, nw, nh) || !img || !bf || !f32 || !err || !out || pitch < w)
@@ -295,7 +295,7 @@ cudaError_t launch_rescale_gemm(const float* img, long long pitch, int w, int h,
     a.n_conv = a.cb * kRsgChunks;
     a.n_wmap = a.cb * ((nw + kRsgRowsPerBlock - 1) / kRsgRowsPerBlock);
     const int n_kmap = a.kcb * ((nh + kRsgRowsPerBlock - 1) / kRsgRowsPerBlock);
-    k_rsg_prep<<<a.n_conv + a.n_wmap + n_kmap, 256, 0, st>>>(a);
+    k_rsg_prep<<<have_maps ? a.n_conv : a.n_conv + a.n_wmap + n_kmap, 256, 0, st>>>(a);
     k_rsg_u<<<a.cb, 256, 0, st>>>(img, pitch, part, w, h, nw, uc, bias);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
