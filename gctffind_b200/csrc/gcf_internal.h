@@ -327,7 +327,8 @@ cudaError_t launch_umma_gemm(const __nv_bfloat16* A, long long lda, const __nv_b
                              GemmArgs g, int bn, int stages, int ntiles, cudaStream_t st);
 // The same product by one persistent CTA per SM over all tiles, the
 // accumulator double-buffered in tensor memory (pairs 256 x 3/4, 128 x 4/6,
-// 64 x 4, 32 x 4).
+// 64 x 4, 32 x 4); large products of the 256-wide tile by pairs of CTAs on
+// 256 x 256 tiles.
 cudaError_t launch_umma_gemm_persistent(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B,
                                         long long ldb, GemmArgs g, int bn, int stages, int ntiles, cudaStream_t st);
 

@@ -528,6 +528,214 @@ k_umma_gemm_persistent(const __grid_constant__ CUtensorMap ta, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------
+// Pair variant for large products (the rescale's): a cluster of two CTAs on
+// one 256 x 256 tile (tcgen05.mma.cta_group::2).  Each CTA stages its half of
+// A (128 rows) and of B (128 columns), so a K slice is 32 KB per CTA instead
+// of 48 KB: two thirds of the shared-memory fills and reads per multiply-add,
+// and six slices in flight instead of four.  The leader's MMA thread issues
+// for both; either CTA's tensor memory holds 128 rows of the accumulator,
+// double-buffered as in k_umma_gemm_persistent, whose warp roles, order of
+// the sums and bounded waits are kept.  Both CTAs' loads signal the leader's
+// "slice loaded" barrier (no multicast: each loads its own part); "slice
+// consumed" and "accumulator full" are committed to both CTAs; the epilogue
+// warps of both arrive at the leader's "accumulator drained".
+//
+// Bound: the tensor pipe.  8192^3: 886 -> 776 us (1241 -> 1417 TFLOP/s; the
+// measured library peak is 1686).  Same results, bit for bit.
+constexpr int kQThreads = 192;
+
+template <int STAGES>
+struct QGemmSmem {
+    static constexpr int kBN = 256;                  // columns of the pair's tile
+    static constexpr int kHalf = kBM * kBK * 2;      // one CTA's part of A, or of B, per stage: 16 KB
+    static constexpr int kStage = 2 * kHalf;
+    static constexpr int kEpi = 4 * 4096;
+    static constexpr int kBars = 1024;
+    static constexpr int kBytes = 1024 + STAGES * kStage + kEpi + kBars;
+};
+
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], "
+        "[%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
+
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// The barrier at the same offset of both CTAs arrives once the MMAs issued so
+// far are done.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar)
+{
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)3)
+        : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync_all()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int STAGES>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQThreads, 1)
+k_umma_gemm_pair(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmArgs g, int ntiles)
+{
+    using L = QGemmSmem<STAGES>;
+    constexpr int BN = L::kBN;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sA = smem;
+    unsigned char* sB = smem + STAGES * L::kHalf;
+    unsigned char* sEpi = smem + STAGES * L::kStage;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + L::kEpi);
+    // [0, S): slice loaded (the leader's counts both CTAs' bytes); [S, 2S):
+    // slice consumed; 2S, 2S+1: accumulator b full; 2S+2, 2S+3: accumulator b
+    // drained (the leader's)
+    uint32_t* s_taddr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+    int* s_abort = reinterpret_cast<int*>(s_taddr + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+    const int gn = (g.N + BN - 1) / BN;
+    const int nkb = (g.K + kBK - 1) / kBK;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2 * STAGES + 2; ++i) mbar_init(smem_u32(bars + i), 1);
+        mbar_init(smem_u32(bars + 2 * STAGES + 2), 8);
+        mbar_init(smem_u32(bars + 2 * STAGES + 3), 8);
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_taddr)),
+                     "r"(2 * BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers and tensor memory are set up
+    tc_fence_after();
+    const uint32_t tmem = *s_taddr;
+    volatile int* abort_flag = s_abort;
+
+    if (warp == 0 && lane == 0) {
+        // producer: this CTA's halves
+        int it = 0;
+        for (int t = pair; t < ntiles && !*abort_flag; t += npairs) {
+            const int m0 = (t / gn) * 2 * kBM + (int)rank * kBM, n0 = (t % gn) * BN + (int)rank * (BN / 2);
+            for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int s = it % STAGES;
+                if (it >= STAGES && !mbar_wait(smem_u32(bars + STAGES + s), ((it / STAGES) & 1) ^ 1)) {
+                    atomicExch(g.err, 1);
+                    *abort_flag = 1;
+                    break;
+                }
+                if (*abort_flag) break;
+                if (rank == 0) mbar_expect_tx(smem_u32(bars + s), 2 * L::kStage);
+                const uint32_t fb = map_rank(smem_u32(bars + s), 0);
+                tma_load_2d_pair(smem_u32(sA + s * L::kHalf), &ta, fb, kb * kBK, m0);
+                tma_load_2d_pair(smem_u32(sB + s * L::kHalf), &tb, fb, kb * kBK, n0);
+            }
+        }
+        // on an abort, the loads still in flight land before the pair exits:
+        // a bounded pause (they signal the leader's barriers, which may never
+        // complete), then the cluster barrier below
+        if (*abort_flag) {
+            const uint64_t t0 = global_ns();
+            while (global_ns() - t0 < 20000000ull) __nanosleep(1000);
+        }
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+        // MMA issuer, for both CTAs
+        constexpr uint32_t idesc =
+            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
+        int it = 0, i = 0;
+        for (int t = pair; t < ntiles && !*abort_flag; t += npairs, ++i) {
+            const int b = i & 1, use = i >> 1;
+            if (use > 0 && !mbar_wait(smem_u32(bars + 2 * STAGES + 2 + b), (use - 1) & 1)) {
+                atomicExch(g.err, 4);
+                *abort_flag = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t tacc = tmem + (uint32_t)(b * BN);
+            bool bad = false;
+            for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int s = it % STAGES;
+                if (!mbar_wait(smem_u32(bars + s), (it / STAGES) & 1)) {
+                    atomicExch(g.err, 2);
+                    *abort_flag = 1;
+                    bad = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t da = desc_k128(smem_u32(sA + s * L::kHalf));
+                const uint64_t db = desc_k128(smem_u32(sB + s * L::kHalf));
+#pragma unroll
+                for (int k = 0; k < kBK / kUK; ++k)
+                    umma_pair(tacc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                umma_commit_pair(smem_u32(bars + STAGES + s));
+            }
+            umma_commit_pair(smem_u32(bars + 2 * STAGES + b));   // accumulator b complete (or abandoned)
+            if (bad) break;
+        }
+    } else if (warp >= 2) {
+        // epilogue warps: this CTA's 128 rows
+        const int q = warp & 3;
+        int i = 0;
+        for (int t = pair; t < ntiles; t += npairs, ++i) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+            const int b = i & 1, use = i >> 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(bars + 2 * STAGES + b), use & 1))) {
+                if (lane == 0) {
+                    atomicExch(g.err, 3);
+                    *abort_flag = 1;
+                }
+                break;
+            }
+            tc_fence_after();
+            const int m0 = (t / gn) * 2 * kBM + (int)rank * kBM, n0 = (t % gn) * BN;
+            const bool wr = !__any_sync(0xffffffffu, *abort_flag != 0);
+            store_accumulator<BN>(g, tmem + (uint32_t)(b * BN), q, lane, m0, n0, sEpi + (warp - 2) * 4096, wr);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(
+                                 map_rank(smem_u32(bars + 2 * STAGES + 2 + b), 0))
+                             : "memory");
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync_all();   // neither CTA leaves while the other may still signal or read it
+    tc_fence_after();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Host side: tensor maps through the driver entry point (no -lcuda), kernel
 // attributes, launch.
 namespace {
@@ -602,9 +810,40 @@ cudaError_t launch_pbn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
     return cudaGetLastError();
 }
 
+template <int STAGES>
+cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, cudaStream_t st)
+{
+    using L = QGemmSmem<STAGES>;
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(k_umma_gemm_pair<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+    });
+    if (attr_err != cudaSuccess) return attr_err;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int tiles = ((g.M + 2 * kBM - 1) / (2 * kBM)) * ((g.N + L::kBN - 1) / L::kBN);
+    const int pairs = std::max(1, std::min(tiles, sms / 2));
+    k_umma_gemm_pair<STAGES><<<2 * pairs, kQThreads, L::kBytes, st>>>(ta, tb, g, tiles);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 int umma_tile_n_supported(int bn) { return bn == 32 || bn == 64 || bn == 128 || bn == 256; }
+
+// Products of the 128 x 256 tile on the whole grid that fill the chip with
+// 256 x 256 tiles go to CTA pairs: 3412 x 3413 x 4097 (196 such tiles on 74
+// pairs) 108 -> 96 us, 4092 x 4800 x 5760 220 -> 182 us.  With fewer tiles
+// than two per pair the larger tile leaves SMs idle, and a short K (fewer
+// slices than both rings hold) gains nothing from the deeper ring.
+static bool takes_pairs(const GemmArgs& g, int bn, int sms)
+{
+    const long long tiles = (long long)((g.M + 255) / 256) * ((g.N + 255) / 256);
+    return bn == 256 && !g.tiles && tiles >= sms && g.K >= 1024;
+}
 
 cudaError_t launch_umma_gemm_persistent(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B,
                                         long long ldb, GemmArgs g, int bn, int stages, int ntiles, cudaStream_t st)
@@ -615,7 +854,15 @@ cudaError_t launch_umma_gemm_persistent(const __nv_bfloat16* A, long long lda, c
     if (g.tiles && ntiles <= 0) return cudaSuccess;
     g.vec4 = (g.D && ((uintptr_t)g.D & 15) == 0 && g.ldd % 4 == 0) ? 1 : 0;
     CUtensorMap ta, tb;
-    cudaError_t e;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (takes_pairs(g, bn, sms)) {
+        if ((e = make_map(&ta, A, g.M, g.K, lda, kBM)) != cudaSuccess) return e;
+        if ((e = make_map(&tb, B, g.N, g.K, ldb, kBM)) != cudaSuccess) return e;
+        return launch_pair<6>(ta, tb, g, st);
+    }
     if ((e = make_map(&ta, A, g.M, g.K, lda, kBM)) != cudaSuccess) return e;
     if ((e = make_map(&tb, B, g.N, g.K, ldb, bn)) != cudaSuccess) return e;
     switch (bn * 10 + stages) {
