@@ -1174,12 +1174,14 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     // Candidate blocks per (chunk, job) of the line searches (at most 4
     // blocks of 16 but for wide phase ranges): one block loops over the
     // candidate blocks it is given, reusing its pixels, so with many jobs
-    // fewer y-blocks (enough for about four CTAs per SM: 8 jobs 2040 us
-    // against 2164 us with enough for six) do the same work without the
-    // blocks that find no candidates and exit.
+    // fewer y-blocks do the same work without the blocks that find no
+    // candidates and exit.  Enough for about four CTAs per SM where the last
+    // CTA ends a step (8 jobs 2040 us against 2164 us with enough for six),
+    // two where every CTA does (4 jobs 1203 us against 1368 us with four).
     const long long per_y = (long long)nj * max_chunks;
-    const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (4LL * ctx->n_sms + per_y - 1) / per_y));
     const int last_ends = eval_last_ends(per_y, ctx->n_sms);
+    const long long want = (last_ends ? 4LL : 2LL) * ctx->n_sms;
+    const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (want + per_y - 1) / per_y));
     for (int k = 0; k < steps; ++k) {
         int cb = (k == 0) ? 1 : (k == 1 && any_grid) ? (kMaxCand / kEvalCB + 3) / 4 : line_cb;
         CK(launch_eval2d(a, k0 + k, cb, max_band, last_ends, ctx->st));

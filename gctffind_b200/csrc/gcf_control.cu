@@ -37,21 +37,38 @@ struct Cand {
 
 // Candidate -> (mean px, sigma*cos 2a, sigma*sin 2a, add/pi); mCorrelate +
 // GCalcCTF2D::DoIt (FindCTF/CFindDefocus2D.cpp:363-380, FindCTF/GCalcCTF2D.cu:117-132).
-__device__ float4 cand_params(const Cand& c, const PixOptics& o)
+__device__ __forceinline__ float cand_mean(const Cand& c, const PixOptics& o)
 {
-    float ph = c.phase * kD2R2D;
-    float az = c.ang * kD2R2D;
     float dmin = c.dfmean * (1.0f - c.ast) / o.px;
     float dmax = c.dfmean * (1.0f + c.ast) / o.px;
-    float mean = 0.5f * (dmin + dmax);
-    float sig = 0.5f * (dmax - dmin);
+    return 0.5f * (dmin + dmax);
+}
+__device__ __forceinline__ float cand_sigma(const Cand& c, const PixOptics& o)
+{
+    float dmin = c.dfmean * (1.0f - c.ast) / o.px;
+    float dmax = c.dfmean * (1.0f + c.ast) / o.px;
+    return 0.5f * (dmax - dmin);
+}
+__device__ __forceinline__ double cand_angle2(const Cand& c)
+{
+    float az = c.ang * kD2R2D;
+    return 2.0 * (double)az;
+}
+__device__ __forceinline__ float cand_phase(const Cand& c, const PixOptics& o)
+{
+    float ph = c.phase * kD2R2D;
     float add = o.amp_phase + ph;
-    double a2 = 2.0 * (double)az;
+    return (float)((double)add / kPi);
+}
+__device__ float4 cand_params(const Cand& c, const PixOptics& o)
+{
+    const float sig = cand_sigma(c, o);
+    const double a2 = cand_angle2(c);
     float4 q;
-    q.x = mean;
+    q.x = cand_mean(c, o);
     q.y = (float)((double)sig * cos(a2));
     q.z = (float)((double)sig * sin(a2));
-    q.w = (float)((double)add / kPi);
+    q.w = cand_phase(c, o);
     return q;
 }
 
@@ -531,7 +548,9 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 //    step the line steps of a single search took 13-16 us each and 1-3 us of
 //    launch gap, of which 9000-12000 cycles were the state machine, on an SM
 //    that had last run that code many steps ago.  Run by all CTAs at every
-//    step it stays in their instruction caches: 10 us per step.
+//    step it stays in their instruction caches, the state and the sums are
+//    read at once, and four warps share a candidate's slow parts (double sine,
+//    cosine and divisions): 8.5 us per step.
 //  * many CTAs (last_ends = 1): the same work in every CTA would cost more
 //    than it saves (96 searches at once: 18.6 ms against 16.1 ms), so the
 //    job's last CTA to finish (an arrival counter, no waiting) ends the step
@@ -539,6 +558,8 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 //
 // In both, the astigmatism grid's 2601 candidates are summed by the last CTA
 // of each candidate block y, in parallel over y, not by one CTA.
+constexpr int kFastCand = 64;   // candidates whose sums are read before their count is known
+
 __global__ void __launch_bounds__(kEvalThreads, 3)
 k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const BandDev* __restrict__ bands,
          const float* __restrict__ band_spec, const int2* __restrict__ spec_off, const double* __restrict__ sum_ss,
@@ -593,29 +614,95 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
     // open: a step of this search is pending; fresh: its first, with no
     // candidates yet
     const int* const jw = reinterpret_cast<const int*>(jin + j);
-    int kind = __ldcg(&jin[j].step), ncand = __ldcg(&jin[j].ncand);
-    const bool open = kind != STEP_DONE, fresh = __ldcg(&jin[j].fresh) != 0;
-    if (!last_ends || fresh || !open) {
-        if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = __ldcg(jw + threadIdx.x);
+    int kind, ncand;
+    bool fresh;
+    if (!last_ends) {
+        // the state and the first kFastCand candidates' sums come in together
+        // (whether that many are there or not), four threads per candidate
+        const int u = threadIdx.x & (kFastCand - 1), q = threadIdx.x / kFastCand;
+        constexpr int G = kEvalThreads / kFastCand;
+        const double2* p = pin + (size_t)j * max_chunks * kLineCand + u;
+        const int word = threadIdx.x < kJobWords ? __ldcg(jw + threadIdx.x) : 0;
+        double cs = 0.0, cc = 0.0;
+#pragma unroll 10
+        for (int k = q; k < nchunk; k += G) {
+            const double2 v = __ldcg(p + (size_t)k * kLineCand);
+            cs += v.x;
+            cc += v.y;
+        }
+        if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = word;
+        shs[threadIdx.x] = make_double2(cs, cc);
         __syncthreads();
-        if (open) {
-            ArgMax m{0.0f, -1};
-            if (!fresh && ncand > kLineCand) {   // the launch before chose
-                const float2 q = __ldcg(reinterpret_cast<const float2*>(best_in + j));
-                m = ArgMax{q.x, __float_as_int(q.y)};
-            } else if (!fresh) {
-                m = reduce_candidates(ncand, 0, 1, ncand, pin + (size_t)j * max_chunks * kLineCand, kLineCand, nchunk,
-                                      sum_ss[j], shs, shm, &s_cc0);
+        kind = sJ.step;
+        ncand = sJ.ncand;
+        fresh = sJ.fresh != 0;
+        if (kind != STEP_DONE) {
+            ArgMax m{(float)-1e20, -1};
+            if (fresh) {
+                __syncthreads();   // every thread has read the state that thread 0 changes below
+            } else if (ncand > kLineCand) {   // the launch before chose
+                __syncthreads();
+                const float2 b = __ldcg(reinterpret_cast<const float2*>(best_in + j));
+                m = ArgMax{b.x, __float_as_int(b.y)};
+            } else if (ncand > kFastCand) {
+                m = reduce_candidates(ncand, 0, 1, ncand, p - u, kLineCand, nchunk, sum_ss[j], shs, shm, &s_cc0);
+            } else {
+                static_assert(kFastCand == 64, "two warps choose");
+                if (threadIdx.x < kFastCand) {
+                    if (u < ncand) {
+#pragma unroll
+                        for (int g = 1; g < G; ++g) {
+                            cs += shs[u + g * kFastCand].x;
+                            cc += shs[u + g * kFastCand].y;
+                        }
+                        const double d = sqrt(cc * sum_ss[j]);
+                        const float v = (d == 0.0) ? 0.0f : (float)(cs / d);   // GCC2D mGCalc1D
+                        if (u == 0) s_cc0 = v;
+                        if (v > m.v) m = ArgMax{v, u};
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        ArgMax t;
+                        t.v = __shfl_xor_sync(0xffffffffu, m.v, o);
+                        t.i = __shfl_xor_sync(0xffffffffu, m.i, o);
+                        m = better(m, t);
+                    }
+                    if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = m;
+                }
+                __syncthreads();
+                m = better(shm[0], shm[1]);
             }
             if (threadIdx.x == 0) next_step(sJ, !fresh, ncand, m, s_cc0, s_cval);
             __syncthreads();
             kind = sJ.step;
             ncand = sJ.ncand;
         }
-        if ((!last_ends || !open) && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
+        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
             reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
-        if (kind == STEP_DONE) return;
+    } else {
+        kind = __ldcg(&jin[j].step);
+        ncand = __ldcg(&jin[j].ncand);
+        fresh = __ldcg(&jin[j].fresh) != 0;
+        if (fresh || kind == STEP_DONE) {
+            if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = __ldcg(jw + threadIdx.x);
+            __syncthreads();
+            if (kind == STEP_DONE) {   // passed on; a fresh state is written by the step's last CTA
+                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
+                    reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
+                return;
+            }
+            if (threadIdx.x == 0) next_step(sJ, false, 0, ArgMax{0.0f, -1}, 0.0f, s_cval);
+            __syncthreads();
+            kind = sJ.step;
+            ncand = sJ.ncand;
+            if (kind == STEP_DONE) {
+                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
+                    reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
+                return;
+            }
+        }
     }
+    if (kind == STEP_DONE) return;
     const int cand_blocks = (ncand + kEvalCB - 1) / kEvalCB;
     if ((int)blockIdx.y >= cand_blocks) return;
     // steps whose candidates move one parameter by a fixed step: the mean
@@ -629,13 +716,40 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
     // candidate blocks y, y + gridDim.y, ... so any candidate count is covered
     for (int c0 = blockIdx.y * kEvalCB; c0 < ncand && nchunk > 0; c0 += gridDim.y * kEvalCB) {
         __syncthreads();
-        if (threadIdx.x < kEvalCB) {
-            const int c = c0 + threadIdx.x;
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (c < ncand)
-                q = last_ends && !fresh ? __ldcg(cand + (size_t)j * kMaxCand + c)
-                                        : cand_params(cand_of(sJ, c, s_cval), sJ.o);
-            sq[threadIdx.x] = q;
+        if (last_ends && !fresh) {
+            if (threadIdx.x < kEvalCB) {
+                const int c = c0 + threadIdx.x;
+                sq[threadIdx.x] =
+                    c < ncand ? __ldcg(cand + (size_t)j * kMaxCand + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        } else {
+            // cand_params of the block's candidates, a warp for each slow part
+            const int i = threadIdx.x & 31, part = threadIdx.x >> 5;
+            double* const cs2 = reinterpret_cast<double*>(shs);   // cos, sin of twice the angle
+            if (part < 4 && i < kEvalCB && c0 + i < ncand) {
+                const Cand c = cand_of(sJ, c0 + i, s_cval);
+                if (part == 0) {
+                    sq[i].x = cand_mean(c, sJ.o);
+                    sq[i].y = cand_sigma(c, sJ.o);
+                } else if (part == 1) {
+                    cs2[i] = cos(cand_angle2(c));
+                } else if (part == 2) {
+                    cs2[kEvalCB + i] = sin(cand_angle2(c));
+                } else {
+                    sq[i].w = cand_phase(c, sJ.o);
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x < kEvalCB) {
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c0 + (int)threadIdx.x < ncand) {
+                    q = sq[threadIdx.x];
+                    const double sig = q.y;
+                    q.y = (float)(sig * cs2[threadIdx.x]);
+                    q.z = (float)(sig * cs2[kEvalCB + threadIdx.x]);
+                }
+                sq[threadIdx.x] = q;
+            }
         }
         __syncthreads();
         float acs[kEvalCB], acc[kEvalCB];
@@ -1314,10 +1428,10 @@ k_table_search(TableArgs A)
 
 }  // namespace
 
-// 1 search (41 CTAs per candidate block): 775 us with every CTA ending the
-// step before, 860 us with the last CTA ending each; 2 (82 CTAs) 995 and
-// 1040; 4 (164 CTAs) 1454 and 1369; 8 (328 CTAs) 2375 and 2042.
-int eval_last_ends(long long ctas, int sms) { return ctas > sms ? 1 : 0; }
+// 1 search (41 CTAs per candidate block): 682 us with every CTA ending the
+// step before, 860 us with the last CTA ending each; 4 (164 CTAs) 1203 and
+// 1378; 8 (328 CTAs) 2041 and 2055; 12 (492 CTAs) 2845 and 2717.
+int eval_last_ends(long long ctas, int sms) { return ctas > 2LL * sms ? 1 : 0; }
 
 cudaError_t launch_eval2d(const EvalArgs& a, int k, int cand_blocks, int max_band_n, int last_ends,
                           cudaStream_t st)
