@@ -428,8 +428,14 @@ void launch_col2im_3s2_relu(const float* dcols, const __nv_bfloat16* y, int B, i
 void launch_relu_bwd(const float* dy, long long ldy, const __nv_bfloat16* y, long long ldyy, int rows, int n,
                      __nv_bfloat16* dz, long long ldz, cudaStream_t st);
 void launch_concat(const __nv_bfloat16* x1, const __nv_bfloat16* y4, int B, __nv_bfloat16* h0, cudaStream_t st);
-void launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows, int nout,
-                  int nin, float* dw, float* db, cudaStream_t st);
+// Weight and bias gradients of a layer (dw: nout x nin, then nout biases);
+// x and dz rows 16-byte aligned with ldz a multiple of 8 (columns nout .. ldz
+// zero); scratch: kWgSlices x (the largest tile's and bias's floats), see
+// wgrad_scratch_floats
+constexpr int kWgSlices = 148;
+constexpr size_t wgrad_scratch_floats() { return (size_t)kWgSlices * 32 * (288 + 1) + 256 * (2304 + 1) * 2; }
+cudaError_t launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows,
+                         int nout, int nin, float* scratch, float* dw, cudaStream_t st);
 void launch_mse(const float* pred, long long ldp, const float* target, int B, float* loss, __nv_bfloat16* dpred,
                 cudaStream_t st);
 void launch_adam(float* w, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,

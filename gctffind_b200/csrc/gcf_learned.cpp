@@ -74,6 +74,7 @@ struct NnNet {
     std::vector<Layer> L = layers();
     size_t np = 0;
     Buf<float> w, g, m, v;                 // masters, gradients, Adam moments
+    Buf<float> wg;                         // slices of a layer's weight gradient
     Buf<__nv_bfloat16> wb, wt;             // BF16 copies
     std::vector<size_t> wb_off, wt_off;
     int steps = 0;
@@ -273,48 +274,47 @@ static cudaError_t layer_dx(NnNet* n, int li, const __nv_bfloat16* dz, long long
     return launch_umma_gemm(dz, ldz, n->wt.p + n->wt_off[li], l.ldt, g, bn, bn == 256 ? 3 : 4, 0, st);
 }
 
-static void layer_dw(NnNet* n, int li, const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* in, int rows,
-                     cudaStream_t st)
+static cudaError_t layer_dw(NnNet* n, int li, const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* in,
+                            int rows, cudaStream_t st)
 {
     const Layer& l = n->L[li];
-    float* dw = n->g.p + l.off;
-    launch_wgrad(dz, ldz, in, l.in, rows, l.out, l.in, dw, dw + (size_t)l.out * l.in, st);
+    return launch_wgrad(dz, ldz, in, l.in, rows, l.out, l.in, n->wg.p, n->g.p + l.off, st);
 }
 
 cudaError_t nn_backward(NnNet* n, const float* target, int B, float* loss, cudaStream_t st)
 {
     if (B > n->B) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(n->g.p, 0, n->np * sizeof(float), st);
+    cudaError_t e = n->wg.ensure(wgrad_scratch_floats());
     if (e != cudaSuccess) return e;
     launch_mse(n->pred.p, kNnPredPitch, target, B, loss, n->dpred.p, st);
     // fc3 (linear): dz = dpred
-    layer_dw(n, 6, n->dpred.p, 8, n->h2.p, B, st);
+    if ((e = layer_dw(n, 6, n->dpred.p, 8, n->h2.p, B, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 6, n->dpred.p, 8, B, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_relu_bwd(n->fbuf.p, 128, n->h2.p, 128, B, 128, n->dz_a.p, 128, st);
     // fc2
-    layer_dw(n, 5, n->dz_a.p, 128, n->h1.p, B, st);
+    if ((e = layer_dw(n, 5, n->dz_a.p, 128, n->h1.p, B, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 5, n->dz_a.p, 128, B, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_relu_bwd(n->fbuf.p, 256, n->h1.p, 256, B, 256, n->dz_b.p, 256, st);
     // fc1: the input gradient of its conv4 part only (the profile is an input)
-    layer_dw(n, 4, n->dz_b.p, 256, n->h0.p, B, st);
+    if ((e = layer_dw(n, 4, n->dz_b.p, 256, n->h0.p, B, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 4, n->dz_b.p, 256, B, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_relu_bwd(n->fbuf.p + 256, 2304, n->y4.p, 2048, B, 2048, n->dz_a.p, 2048, st);
     // conv4: dz_a is [B*64][32]
-    layer_dw(n, 3, n->dz_a.p, 32, n->cols4.p, B * 64, st);
+    if ((e = layer_dw(n, 3, n->dz_a.p, 32, n->cols4.p, B * 64, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 3, n->dz_a.p, 32, B * 64, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_col2im_3s2_relu(n->fbuf.p, n->y3.p, B, 16, 16, 32, n->dz_b.p, st);
     // conv3
-    layer_dw(n, 2, n->dz_b.p, 32, n->cols3.p, B * 256, st);
+    if ((e = layer_dw(n, 2, n->dz_b.p, 32, n->cols3.p, B * 256, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 2, n->dz_b.p, 32, B * 256, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_col2im_3s2_relu(n->fbuf.p, n->y2.p, B, 32, 32, 32, n->dz_a.p, st);
     // conv2
-    layer_dw(n, 1, n->dz_a.p, 32, n->cols2.p, B * 1024, st);
+    if ((e = layer_dw(n, 1, n->dz_a.p, 32, n->cols2.p, B * 1024, st)) != cudaSuccess) return e;
     if ((e = layer_dx(n, 1, n->dz_a.p, 32, B * 1024, n->fbuf.p, st)) != cudaSuccess) return e;
     launch_col2im_3s2_relu(n->fbuf.p, n->y1.p, B, 64, 64, 16, n->dz_b.p, st);
     // conv1 (its input needs no gradient): its im2col rows for the weight
     // gradient (the forward reads the input directly)
     launch_im2col_p4(n->x2, B, n->cols1.p, st);
-    layer_dw(n, 0, n->dz_b.p, 16, n->cols1.p, B * 4096, st);
+    if ((e = layer_dw(n, 0, n->dz_b.p, 16, n->cols1.p, B * 4096, st)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
 

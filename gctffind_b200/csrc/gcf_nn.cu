@@ -14,8 +14,8 @@
 //   fc1 [x1, conv4] 2304 -> 256 (ReLU), fc2 256 -> 128 (ReLU), fc3 128 -> 3
 //   outputs: (mean defocus - 22500) / 10000, astigmatism / 1000 * (cos 2a, sin 2a)
 // Forward layers and the input gradients run as tensor-core products
-// (im2col rows x weights); weight gradients are reductions over the batch's
-// rows (long K, few outputs) done here on the FP32 pipe.
+// (im2col rows x weights); weight gradients are contractions over the batch's
+// rows (long K, few outputs) done here with mma.sync and FP64 sums of slices.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -389,33 +389,41 @@ __global__ void k_im2col_3s2(const __nv_bfloat16* __restrict__ x, int B, int H, 
 // Gradient of a 3 x 3 stride-2 pad-1 layer's input from its im2col
 // gradient dcols (FP32, [B*OH*OW][9C]), times the ReLU derivative of the
 // input activation y (> 0), as BF16 [B][H][W][C].
+// Four channels per thread, 16-byte loads: 88 us per step of 256 samples,
+// near its bytes' time.  One thread per value took 327 us, bound by its index
+// arithmetic.
 __global__ void k_col2im_3s2_relu(const float* __restrict__ dcols, const __nv_bfloat16* __restrict__ y, int B,
                                   int H, int W, int C, __nv_bfloat16* __restrict__ dz)
 {
-    const int OH = H / 2, OW = W / 2, K = 9 * C;
-    const long long n = (long long)B * H * W * C;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        const long long r = i / C;
-        const int xx = (int)(r % W), yy = (int)((r / W) % H), b = (int)(r / ((long long)W * H));
-        float s = 0.0f;
-        if (bf(y[i]) > 0.0f) {
-            // output rows oy with 2 oy - 1 + ky = yy, ky in 0..2
-            for (int ky = 0; ky < 3; ++ky) {
-                const int t = yy + 1 - ky;
-                if (t < 0 || (t & 1)) continue;
-                const int oy = t >> 1;
-                if (oy >= OH) continue;
-                for (int kx = 0; kx < 3; ++kx) {
-                    const int u = xx + 1 - kx;
-                    if (u < 0 || (u & 1)) continue;
-                    const int ox = u >> 1;
-                    if (ox >= OW) continue;
-                    s += dcols[(((size_t)b * OH + oy) * OW + ox) * K + (ky * 3 + kx) * C + c];
-                }
+    const int OH = H / 2, OW = W / 2, K = 9 * C, C4 = C / 4;
+    const int n = B * H * W * C4;   // < 2^31: B <= 4096
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int c = i % C4 * 4, r = i / C4;
+        const int xx = r % W, yb = r / W, yy = yb % H, b = yb / H;
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        // output rows oy with 2 oy - 1 + ky = yy, ky in 0..2
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+            const int t = yy + 1 - ky, oy = t >> 1;
+            if (t < 0 || (t & 1) || oy >= OH) continue;
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx) {
+                const int u = xx + 1 - kx, ox = u >> 1;
+                if (u < 0 || (u & 1) || ox >= OW) continue;
+                const float4 v = __ldg(reinterpret_cast<const float4*>(
+                    dcols + (((size_t)b * OH + oy) * OW + ox) * K + (ky * 3 + kx) * C + c));
+                s[0] += v.x;
+                s[1] += v.y;
+                s[2] += v.z;
+                s[3] += v.w;
             }
         }
-        dz[i] = __float2bfloat16_rn(s);
+        const uint2 yq = __ldg(reinterpret_cast<const uint2*>(y) + i);
+        const __nv_bfloat16* yv = reinterpret_cast<const __nv_bfloat16*>(&yq);
+        __nv_bfloat16 q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = __float2bfloat16_rn(bf(yv[k]) > 0.0f ? s[k] : 0.0f);
+        reinterpret_cast<uint2*>(dz)[i] = *reinterpret_cast<const uint2*>(q);
     }
 }
 
@@ -442,40 +450,184 @@ __global__ void k_concat(const __nv_bfloat16* __restrict__ x1, const __nv_bfloat
     }
 }
 
-// Weight and bias gradients dW[o][k] += sum_r dz[r][o] x[r][k],
-// db[o] += sum_r dz[r][o]: 32 x 32 output tiles, each CTA a slice of rows
-// staged through shared memory, FP32 sums, atomics into dW.
-__global__ void __launch_bounds__(256)
-k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16* __restrict__ x, long long ldx,
-        int rows, int nout, int nin, int rows_per_cta, float* __restrict__ dw, float* __restrict__ db)
+// Weight and bias gradients dW[o][k] = sum_r dz[r][o] x[r][k],
+// db[o] = sum_r dz[r][o] of a layer, in two kernels: k_wgrad sums slices of
+// rows, k_wgrad_sum adds the slices in order (deterministic, no atomics).
+//
+// Bound: reading x and dz once (205 MB per step of 256 samples, 32 us); the
+// products are a contraction over up to a million rows with at most 32 x 288
+// outputs, far too few for a tcgen05 tile to pay for its staging, so they run
+// as mma.sync m16n8k16 on fragments that ldmatrix transposes out of shared
+// memory.  The scalar kernel staged 32 x 32 tiles as floats, read x once per 32
+// outputs and dz once per 32 inputs, and added its slices with atomics: 931 us
+// per step of 256 samples; these two kernels take 132 us.  Relative error
+// against FP64 sums: 1.1e-7 for a million rows x 16 columns (4.6e-7 before),
+// 7.5e-8 for 262144 x 144 (2.6e-7), 3.6e-8 for 6400 x 288 (1.1e-7).
+//
+// A CTA takes 32 outputs x KT columns and a slice of rows, in chunks through
+// a ring of kWgStages shared-memory stages (cp.async, 16 bytes).  Its eight
+// warps split the KT columns into groups of CW and the rows of a chunk among
+// the warps of a group.  Products are exact in FP32; a warp's tensor-core sums
+// are added to FP32 registers every kWgFlush chunks, so that no long chain
+// keeps the tensor core's truncation.
+constexpr int kWgStages = 4, kWgFlush = 4;
+
+template <int KT_>
+struct WgShape {
+    static constexpr int KT = KT_;
+    static constexpr int CW = KT >= 72 ? 72 : KT;          // columns per warp
+    static constexpr int CG = KT / CW, RG = 8 / CG;        // column groups, warps per group
+    static constexpr int ROWS = KT >= 72 ? 64 : 256;       // rows per chunk
+    static constexpr int STEPS = ROWS / RG / 16;           // k16 steps per warp and chunk
+    static constexpr int NT = CW / 8;                      // n8 tiles per warp
+    static constexpr int XP = KT + 8, ZP = 40;             // row pitches (BF16): an odd number of 16 bytes
+    static constexpr size_t STAGE = (size_t)ROWS * (XP + ZP) * 2;
+    static constexpr size_t SMEM = kWgStages * STAGE;
+    static_assert(STEPS >= 1 && RG * STEPS * 16 == ROWS && CG * CW == KT, "shape");
+    static_assert(STAGE * kWgStages >= (size_t)RG * 32 * KT * 4, "the warps' sums fit the ring");
+};
+
+__device__ __forceinline__ uint32_t nn_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// 16 bytes to shared memory, zeros where !ok
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok)
 {
-    __shared__ float sz[32][33], sx[32][33];
-    const int o0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+template <class S>
+__global__ void __launch_bounds__(256, 1)
+k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16* __restrict__ x, long long ldx,
+        int rows, int nout, int nin, int rows_per_cta, float* __restrict__ part, float* __restrict__ part_b)
+{
+    extern __shared__ __align__(16) unsigned char wsm[];
+    __shared__ float sb[8][32];
+    const int k0 = blockIdx.x * S::KT, o0 = blockIdx.y * 32;
     const int r0 = blockIdx.z * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 8 row groups
-    float acc[4] = {0, 0, 0, 0}, bacc = 0.0f;
-    for (int rb = r0; rb < r1; rb += 32) {
-        for (int q = ty; q < 32; q += 8) {
-            const int r = rb + q;
-            sz[q][tx] = (r < r1 && o0 + tx < nout) ? bf(dz[(size_t)r * ldz + o0 + tx]) : 0.0f;
-            sx[q][tx] = (r < r1 && k0 + tx < nin) ? bf(x[(size_t)r * ldx + k0 + tx]) : 0.0f;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cg = warp / S::RG, rg = warp % S::RG;
+    const int nch = (r1 - r0 + S::ROWS - 1) / S::ROWS;
+    auto xs = [&](int st) { return reinterpret_cast<__nv_bfloat16*>(wsm + st * S::STAGE); };
+    auto zs = [&](int st) { return reinterpret_cast<__nv_bfloat16*>(wsm + st * S::STAGE) + (size_t)S::ROWS * S::XP; };
+    auto fill = [&](int c) {
+        if (c < nch) {
+            const int st = c % kWgStages, rb = r0 + c * S::ROWS;
+            constexpr int XQ = S::KT / 8;   // 16-byte pieces of an x row
+            for (int i = tid; i < S::ROWS * XQ; i += 256) {
+                const int r = i / XQ, q = i - r * XQ;
+                const bool ok = rb + r < r1 && k0 + 8 * q < nin;
+                cp16(nn_smem(xs(st) + (size_t)r * S::XP + 8 * q), ok ? x + (size_t)(rb + r) * ldx + k0 + 8 * q : x, ok);
+            }
+            for (int i = tid; i < S::ROWS * 4; i += 256) {
+                const int r = i >> 2, q = i & 3;
+                const bool ok = rb + r < r1 && o0 + 8 * q < ldz;
+                cp16(nn_smem(zs(st) + (size_t)r * S::ZP + 8 * q), ok ? dz + (size_t)(rb + r) * ldz + o0 + 8 * q : dz, ok);
+            }
         }
-        __syncthreads();
-        // thread (ty, tx): outputs o = o0 + ty + 8 i, k = k0 + tx
-        for (int q = 0; q < 32; ++q) {
-            const float xv = sx[q][tx];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[2][S::NT][4], sum[2][S::NT][4], bsum = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] = fmaf(sz[q][ty + 8 * i], xv, acc[i]);
-            if (blockIdx.x == 0 && ty == 0) bacc += sz[q][tx];
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < S::NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[m][n][i] = sum[m][n][i] = 0.0f;
+    for (int c = 0; c < kWgStages - 1; ++c) fill(c);
+    for (int c = 0; c < nch; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kWgStages - 2) : "memory");
+        __syncthreads();   // chunk c has landed; chunk c - 1 is free
+        fill(c + kWgStages - 1);
+        const __nv_bfloat16 *X = xs(c % kWgStages), *Z = zs(c % kWgStages);
+        if (blockIdx.x == 0)   // bias: this thread's column and eighth of the rows
+            for (int r = warp; r < S::ROWS; r += 8) bsum += bf(Z[r * S::ZP + lane]);
+#pragma unroll
+        for (int t = 0; t < S::STEPS; ++t) {
+            const int rr = (rg * S::STEPS + t) * 16;
+            // A (16 outputs x 16 rows) from [row][output], transposed on load
+            uint32_t af[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int i = lane & 7, mat = lane >> 3;   // matrices: (outputs 0-7, 8-15) x (rows 0-7, 8-15)
+                const uint32_t ad =
+                    nn_smem(Z + (size_t)(rr + (mat >> 1) * 8 + i) * S::ZP + m * 16 + (mat & 1) * 8);
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(af[m][0]), "=r"(af[m][1]), "=r"(af[m][2]), "=r"(af[m][3])
+                             : "r"(ad));
+            }
+#pragma unroll
+            for (int n = 0; n < S::NT; ++n) {
+                // B (16 rows x 8 columns) from [row][column], transposed on load
+                uint32_t b0, b1;
+                const uint32_t bd = nn_smem(X + (size_t)(rr + (lane & 15)) * S::XP + cg * S::CW + n * 8);
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+                             : "=r"(b0), "=r"(b1)
+                             : "r"(bd));
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+                    asm volatile(
+                        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                        "{%8, %9}, {%0, %1, %2, %3};"
+                        : "+f"(acc[m][n][0]), "+f"(acc[m][n][1]), "+f"(acc[m][n][2]), "+f"(acc[m][n][3])
+                        : "r"(af[m][0]), "r"(af[m][1]), "r"(af[m][2]), "r"(af[m][3]), "r"(b0), "r"(b1));
+            }
         }
-        __syncthreads();
-    }
+        if ((c + 1) % kWgFlush == 0 || c + 1 == nch) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int o = o0 + ty + 8 * i, k = k0 + tx;
-        if (o < nout && k < nin) atomicAdd(dw + (size_t)o * nin + k, acc[i]);
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < S::NT; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        sum[m][n][i] += acc[m][n][i];
+                        acc[m][n][i] = 0.0f;
+                    }
+        }
     }
-    if (blockIdx.x == 0 && ty == 0 && o0 + tx < nout && db) atomicAdd(db + o0 + tx, bacc);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // the ring is free: the warps' sums, [row group][output][column]
+    float* ws = reinterpret_cast<float*>(wsm);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < S::NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int o = m * 16 + (lane >> 2) + (i >> 1) * 8, k = cg * S::CW + n * 8 + (lane & 3) * 2 + (i & 1);
+                ws[((size_t)rg * 32 + o) * S::KT + k] = sum[m][n][i];
+            }
+    sb[warp][lane] = bsum;
+    __syncthreads();
+    // part: [slice][output][column] of the whole layer
+    for (int i = tid; i < 32 * S::KT; i += 256) {
+        const int o = o0 + i / S::KT, k = k0 + i % S::KT;
+        if (o >= nout || k >= nin) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int g = 0; g < S::RG; ++g) v += ws[(size_t)g * 32 * S::KT + i];
+        part[((size_t)blockIdx.z * nout + o) * nin + k] = v;
+    }
+    if (blockIdx.x == 0 && tid < 32 && o0 + tid < nout) {
+        float v = 0.0f;
+        for (int w = 0; w < 8; ++w) v += sb[w][tid];
+        part_b[(size_t)blockIdx.z * nout + o0 + tid] = v;
+    }
+}
+
+// dw[i] = sum of the slices' part[z][i], i < n (the bias after the weights),
+// in FP64 in slice order
+__global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ part, const float* __restrict__ part_b,
+                                                   int slices, int nw, int nb, float* __restrict__ dw)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= nw + nb) return;
+    const float* p = i < nw ? part + i : part_b + (i - nw);
+    const size_t st = i < nw ? nw : nb;
+    double s = 0.0;
+#pragma unroll 8
+    for (int z = 0; z < slices; ++z) s += (double)__ldg(p + z * st);
+    dw[i] = (float)s;
 }
 
 // Mean squared error over the 3 outputs: loss (atomic) and
@@ -596,7 +748,7 @@ void launch_im2col_3s2(const __nv_bfloat16* x, int B, int H, int W, int C, __nv_
 void launch_col2im_3s2_relu(const float* dcols, const __nv_bfloat16* y, int B, int H, int W, int C,
                             __nv_bfloat16* dz, cudaStream_t st)
 {
-    k_col2im_3s2_relu<<<grid_for((long long)B * H * W * C, 256), 256, 0, st>>>(dcols, y, B, H, W, C, dz);
+    k_col2im_3s2_relu<<<grid_for((long long)B * H * W * C / 4, 256), 256, 0, st>>>(dcols, y, B, H, W, C, dz);
 }
 
 void launch_relu_bwd(const float* dy, long long ldy, const __nv_bfloat16* y, long long ldyy, int rows, int n,
@@ -610,15 +762,32 @@ void launch_concat(const __nv_bfloat16* x1, const __nv_bfloat16* y4, int B, __nv
     k_concat<<<grid_for((long long)B * 2304, 256), 256, 0, st>>>(x1, y4, B, h0);
 }
 
-void launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows, int nout,
-                  int nin, float* dw, float* db, cudaStream_t st)
+// Row slices of a layer's weight gradient: about one CTA per SM, whole chunks.
+template <class S>
+static cudaError_t wgrad_shape(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows,
+                               int nout, int nin, float* scratch, float* dw, cudaStream_t st)
 {
-    const int gx = (nin + 31) / 32, gy = (nout + 31) / 32;
-    // enough row slices to give every SM a few CTAs
-    int slices = std::max(1, std::min((rows + 255) / 256, (148 * 4 + gx * gy - 1) / (gx * gy)));
-    const int per = ((rows + slices - 1) / slices + 31) / 32 * 32;
+    const int gx = (nin + S::KT - 1) / S::KT, gy = (nout + 31) / 32;
+    int slices = std::max(1, std::min((rows + S::ROWS - 1) / S::ROWS, kWgSlices / (gx * gy)));
+    const int per = ((rows + slices - 1) / slices + S::ROWS - 1) / S::ROWS * S::ROWS;
     slices = (rows + per - 1) / per;
-    k_wgrad<<<dim3(gx, gy, slices), 256, 0, st>>>(dz, ldz, x, ldx, rows, nout, nin, per, dw, db);
+    cudaError_t e = cudaFuncSetAttribute(k_wgrad<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return e;
+    float* part_b = scratch + (size_t)slices * nout * nin;
+    k_wgrad<S><<<dim3(gx, gy, slices), 256, S::SMEM, st>>>(dz, ldz, x, ldx, rows, nout, nin, per, scratch, part_b);
+    const int nw = nout * nin;
+    k_wgrad_sum<<<(nw + nout + 255) / 256, 256, 0, st>>>(scratch, part_b, slices, nw, nout, dw);
+    return cudaGetLastError();
+}
+
+// Column tile by the layer's width: 16 (the first layer), 144 up to that
+// width or where 288 would leave most of a tile empty (256), else 288.
+cudaError_t launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows,
+                         int nout, int nin, float* scratch, float* dw, cudaStream_t st)
+{
+    if (nin <= 16) return wgrad_shape<WgShape<16>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
+    if (nin <= 256) return wgrad_shape<WgShape<144>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
+    return wgrad_shape<WgShape<288>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
 }
 
 void launch_mse(const float* pred, long long ldp, const float* target, int B, float* loss, __nv_bfloat16* dpred,
