@@ -222,7 +222,8 @@ struct gcf_ctx {
     cudaEvent_t rs_fork = nullptr, rs_join = nullptr;   // around the second lane (RescaleLanes)
     DBuf<int> dev_err;            // bounded-wait flag of the tile kernel and the tensor-core
                                   // rescale, checked when results are read
-    DBuf<double> acc, hsum, moments, moments2, tile_sums;
+    DBuf<double> acc, bg_part, moments, moments2, tile_sums;
+    DBuf<unsigned> bg_ticket;
     DBuf<float> lpfull;
     DBuf<float2> lpcmp;
     DBuf<float> raw, ctf0, ctf, radial, band_spec, cc_res, full;
@@ -245,6 +246,7 @@ struct gcf_ctx {
 
     // fused spectrum
     DBuf<float2> tw512;
+    DBuf<float> lp_axis;
     DBuf<FusedImageDesc> f_desc;
     DBuf<int4> f_items;
     DBuf<int> f_first, f_group;
@@ -512,6 +514,10 @@ gcf_status build_tile_tables(gcf_ctx* ctx)
     }
     CK(ctx->tw512.ensure(T));
     CK(cudaMemcpy(ctx->tw512.p, tw.data(), T * sizeof(float2), cudaMemcpyHostToDevice));
+    if (fused_tile_supported(T)) {
+        CK(ctx->lp_axis.ensure(T));
+        CK(launch_lp_axis(ctx->lp_axis.p, 10.0, ctx->st));   // B-factor 10
+    }
     CK(ctx->dev_err.ensure(1));
     CK(cudaMemset(ctx->dev_err.p, 0, sizeof(int)));
     // A copy from pageable memory may return before its DMA lands, and the
@@ -915,7 +921,11 @@ gcf_status spectra_alloc(gcf_ctx* ctx, int nm)
     CK(ctx->raw.ensure(cmp_n * nm));
     CK(ctx->ctf0.ensure(cmp_n * nm));
     CK(ctx->ctf.ensure(cmp_n * nm));
-    CK(ctx->hsum.ensure(cmp_n * nm));
+    CK(ctx->bg_part.ensure(2 * background_blocks(T) * nm));
+    if (ctx->bg_ticket.n < (size_t)nm) {
+        CK(ctx->bg_ticket.ensure(nm));
+        CK(cudaMemsetAsync(ctx->bg_ticket.p, 0, nm * sizeof(unsigned), ctx->st));
+    }
     CK(ctx->moments.ensure(2 * (size_t)nm));
     CK(ctx->lowpassed.ensure(nm));
     CK(ctx->radial.ensure((size_t)cx * nm));
@@ -945,12 +955,9 @@ gcf_status spectra_post(gcf_ctx* ctx, int nm, int first = 0)
     size_t cmp_n = (size_t)cx * T;
     if (nm <= 0) return GCF_OK;
     const size_t o = (size_t)first * cmp_n;
-    launch_bg_horizontal(ctx->raw.p + o, T, nm, ctx->log_spect, ctx->hsum.p + o, ctx->st);
-    CKL();
-    launch_bg_vertical(ctx->raw.p + o, ctx->hsum.p + o, T, nm, ctx->log_spect, ctx->ctf0.p + o, ctx->st);
-    CKL();
-    launch_moments(ctx->ctf0.p + o, (int)cmp_n, nm, ctx->moments.p + 2 * (size_t)first, ctx->st);
-    CKL();
+    CK(launch_background(ctx->raw.p + o, T, nm, ctx->log_spect, ctx->ctf0.p + o,
+                         ctx->bg_part.p + 2 * background_blocks(T) * (size_t)first, ctx->bg_ticket.p + first,
+                         ctx->moments.p + 2 * (size_t)first, ctx->st));
     // CFindCtfBase::mLowpass (FindCTF/CFindCtfBase.cpp:191-219): full
     // spectrum, R2C, B-factor 10 (normalised), C2R, half back.  Tile 512
     // with the hand-written spectrum path: the separable filter on the warp
@@ -958,12 +965,12 @@ gcf_status spectra_post(gcf_ctx* ctx, int nm, int first = 0)
     // variant) batched cuFFT.
     CK(ctx->lpfull.ensure((size_t)nm * T * T));
     if (ctx->impl == GCF_SPECT_FUSED && fused_tile_supported(T)) {
-        CK(launch_lowpass512(ctx->ctf0.p + o, ctx->tw512.p, 10.0, nm, ctx->moments.p + 2 * (size_t)first,
+        CK(launch_lowpass512(ctx->ctf0.p + o, ctx->tw512.p, ctx->lp_axis.p, nm, ctx->moments.p + 2 * (size_t)first,
                              ctx->lpfull.p, ctx->ctf.p + o, ctx->lowpassed.p + first, ctx->st));
         launch_radial(ctx->ctf.p + o, T, nm, ctx->rad_off.p, ctx->rad_pix.p, ctx->radial.p + (size_t)first * cx,
                       ctx->st);
         CKL();
-        ctx->launches += 6;
+        ctx->launches += 4;
         return GCF_OK;
     }
     CK(ctx->lpcmp.ensure((size_t)nm * cx * T));
@@ -992,7 +999,7 @@ gcf_status spectra_post(gcf_ctx* ctx, int nm, int first = 0)
     launch_radial(ctx->ctf.p + o, T, nm, ctx->rad_off.p, ctx->rad_pix.p, ctx->radial.p + (size_t)first * cx,
                   ctx->st);
     CKL();
-    ctx->launches += 7;
+    ctx->launches += 5;
     return GCF_OK;
 }
 
@@ -2025,7 +2032,8 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->dev_err.release();
     ctx->acc.release();
     ctx->tile_sums.release();
-    ctx->hsum.release();
+    ctx->bg_part.release();
+    ctx->bg_ticket.release();
     ctx->lpfull.release();
     ctx->lpcmp.release();
     ctx->moments.release();
@@ -2055,6 +2063,7 @@ void gcf_destroy(gcf_ctx* ctx)
     ctx->d_optics.release();
     ctx->d_counts.release();
     ctx->tw512.release();
+    ctx->lp_axis.release();
     ctx->f_desc.release();
     ctx->f_items.release();
     ctx->f_first.release();

@@ -1389,28 +1389,33 @@ __device__ __forceinline__ void lp_filter_pass(float2 (&v)[16], float2* scr, con
     fft512_warp(v, scr, twl, lane);   // conj(result) = the filtered pair, bin order
 }
 
-__device__ __forceinline__ void lp_setup(float2* twl, float* gk, const float2* twg, double bfactor)
+// The filter's values g(k) / N, once per context.
+__global__ void k_lp_axis(float* __restrict__ g, double bfactor)
+{
+    const double scale = -bfactor / (2.0 * (double)FT * FT);
+    const int k = threadIdx.x, kw = k <= FT / 2 ? k : k - FT;
+    g[k] = (float)(exp(scale * (double)kw * kw) / (double)FT);
+}
+
+__device__ __forceinline__ void lp_setup(float2* twl, float* gk, const float2* twg, const float* axis)
 {
     for (int i = threadIdx.x; i < 16 * 32; i += blockDim.x) twl[i] = twg[((i & 31) * (i >> 5)) & (FT - 1)];
-    const double scale = -bfactor / (2.0 * (double)FT * FT);
-    for (int k = threadIdx.x; k < FT; k += blockDim.x) {
-        const int kw = k <= FT / 2 ? k : k - FT;
-        gk[k] = (float)(exp(scale * (double)kw * kw) / (double)FT);
-    }
+    for (int k = threadIdx.x; k < FT; k += blockDim.x) gk[k] = axis[k];
     __syncthreads();
 }
 
 // Rows: one warp per row pair of the full spectrum built from the half
 // spectrum (GCalcSpectrum::GenFullSpect's mirror, DC at column 256);
-// filtered rows to rowf [m][512][512].
+// filtered rows to rowf [m][512][512], only the columns that the column pass
+// reads (0, 1 and 256 on).
 __global__ void __launch_bounds__(kLpWarps * 32)
-k_lowpass_rows(const float* __restrict__ ctf0, const float2* __restrict__ twg, double bfactor,
+k_lowpass_rows(const float* __restrict__ ctf0, const float2* __restrict__ twg, const float* __restrict__ axis,
                float* __restrict__ rowf)
 {
     __shared__ float2 s_twl[16 * 32];
     __shared__ float s_g[FT];
     __shared__ float2 s_scr[kLpWarps][FSCR];
-    lp_setup(s_twl, s_g, twg, bfactor);
+    lp_setup(s_twl, s_g, twg, axis);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m = blockIdx.y, y0 = 2 * (blockIdx.x * kLpWarps + warp);
     const float* half = ctf0 + (size_t)m * FCX * FT;
@@ -1439,76 +1444,82 @@ k_lowpass_rows(const float* __restrict__ ctf0, const float2* __restrict__ twg, d
     float* ra = rowf + ((size_t)m * FT + y0) * FT;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
+        if (j > 0 && j < 8) continue;
+        if (j == 0 && lane > 1) continue;
         const float2 z = scr[sslot(32 * j + lane)];
         ra[32 * j + lane] = z.x;          // conjugate: a' = Re, b' = -Im
         ra[FT + 32 * j + lane] = -z.y;
     }
 }
 
-// Columns: a CTA takes 32 adjacent columns of the row-filtered spectrum
-// (a 512 x 32 block through shared memory, 128-byte rows), each warp two
-// column pairs; only the columns of the half spectrum are kept: out[y][x] =
-// filtered[y][x + 256] (x < 256) and out[y][256] = filtered[y][0]
-// (CFindCtfBase.cpp:212-218).  Spectra whose background-removed variance is
-// below 1 keep ctf0 (the variance gate of mRemoveBackground,
-// FindCTF/CFindCtfBase.cpp:169-174).
+// Columns: a CTA takes 16 adjacent columns of the row-filtered spectrum (a
+// 512 x 16 block through shared memory, 64-byte rows), one column pair per
+// warp, and writes them back through the same block; only the columns of the
+// half spectrum are kept: out[y][x] = filtered[y][x + 256] (x < 256) and
+// out[y][256] = filtered[y][0] (CFindCtfBase.cpp:212-218).  Spectra whose
+// background-removed variance is below 1 keep ctf0 (the variance gate of
+// mRemoveBackground, FindCTF/CFindCtfBase.cpp:169-174).
+//
+// Bound: latency (one pair's two FFTs per warp) for few spectra, traffic for
+// many.  32 columns per CTA with the results written straight from the lanes
+// (one 4-byte piece of 32 rows per store), the filter's exponentials taken by
+// every block and all 512 columns handed over by the row pass took, both
+// passes together, 25.2 us for one spectrum and 331 us for 256; now
+// 13.1 and 232 us.
+constexpr int kLpCols = 2 * kLpWarps, kLpPitch = kLpCols + 1;
+
 __global__ void __launch_bounds__(kLpWarps * 32)
 k_lowpass_cols(const float* __restrict__ rowf, const float* __restrict__ ctf0, const float2* __restrict__ twg,
-               double bfactor, const double* __restrict__ mom, float* __restrict__ out, int* __restrict__ lowpassed)
+               const float* __restrict__ axis, const double* __restrict__ mom, float* __restrict__ out,
+               int* __restrict__ lowpassed)
 {
-    extern __shared__ float s_blk[];   // [512][33]
+    extern __shared__ float s_blk[];   // [512][kLpPitch]
     __shared__ float2 s_twl[16 * 32];
     __shared__ float s_g[FT];
     __shared__ float2 s_scr[kLpWarps][FSCR];
     const int m = blockIdx.y;
-    // blocks 0..7: columns 256 + 32 b ..; block 8: columns 0 .. 31 (column 0 kept)
-    const int c0 = blockIdx.x < 8 ? FT / 2 + 32 * blockIdx.x : 0;
+    // all but the last block: columns 256 + 16 b ..; the last: columns 0 and 1 (column 0 kept)
+    const bool tail = blockIdx.x == FT / 2 / kLpCols;
+    const int c0 = tail ? 0 : FT / 2 + kLpCols * blockIdx.x;
+    const int ncol = tail ? 2 : kLpCols, nkeep = tail ? 1 : kLpCols, xo = tail ? FT / 2 : c0 - FT / 2;
     const double mean = mom[2 * m], var = mom[2 * m + 1] - mean * mean;
     const bool run = !(var < 1.0);
     if (blockIdx.x == 0 && threadIdx.x == 0) lowpassed[m] = run ? 1 : 0;
-    float* o = out + (size_t)m * FCX * FT;
-    const float* h0 = ctf0 + (size_t)m * FCX * FT;
+    float* o = out + (size_t)m * FCX * FT + xo;
+    const int c = threadIdx.x & (kLpCols - 1), r = threadIdx.x / kLpCols;
+    constexpr int RS = kLpWarps * 32 / kLpCols;   // rows per pass of the block
     if (!run) {
-        for (int i = threadIdx.x; i < FT * 32; i += blockDim.x) {
-            const int y = i >> 5, X = c0 + (i & 31);
-            const int x = X >= FT / 2 ? X - FT / 2 : (X == 0 ? FT / 2 : -1);
-            if (x >= 0) o[(size_t)y * FCX + x] = h0[(size_t)y * FCX + x];
-        }
+        const float* h0 = ctf0 + (size_t)m * FCX * FT + xo;
+        for (int y = r; y < FT && c < nkeep; y += RS) o[(size_t)y * FCX + c] = h0[(size_t)y * FCX + c];
         return;
     }
-    lp_setup(s_twl, s_g, twg, bfactor);
     const float* src = rowf + (size_t)m * FT * FT + c0;
-    for (int i = threadIdx.x; i < FT * 32; i += blockDim.x) {
-        const int y = i >> 5, c = i & 31;
-        s_blk[y * 33 + c] = src[(size_t)y * FT + c];
+    if (c < ncol) {
+#pragma unroll 8
+        for (int y = r; y < FT; y += RS) s_blk[y * kLpPitch + c] = src[(size_t)y * FT + c];
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float2* scr = s_scr[warp];
-    const int npairs = c0 == 0 ? 1 : 2;   // block 8 needs columns 0 and 1 only
-    for (int q = 0; q < npairs; ++q) {
-        const int cl = 2 * (2 * warp + q);   // local column of a; b = cl + 1
-        if (c0 == 0 && warp != 0) break;
+    lp_setup(s_twl, s_g, twg, axis);
+    const int lane = threadIdx.x & 31, cl = 2 * (threadIdx.x >> 5);   // local column of a; b = cl + 1
+    if (cl < ncol) {
         float2 v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const int y = 32 * j + lane;
-            v[j] = make_float2(s_blk[y * 33 + cl], s_blk[y * 33 + cl + 1]);
+            v[j] = make_float2(s_blk[y * kLpPitch + cl], s_blk[y * kLpPitch + cl + 1]);
         }
-        lp_filter_pass(v, scr, s_twl, s_g, lane);
+        lp_filter_pass(v, s_scr[threadIdx.x >> 5], s_twl, s_g, lane);
         const int mm = lane >> 1, p = lane & 1;
-        const int Xa = c0 + cl;
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             const int y = mm + 16 * k + 256 * p;
-            const float2 z = v[P16(k)];
-            if (Xa >= FT / 2) {
-                o[(size_t)y * FCX + (Xa - FT / 2)] = z.x;
-                o[(size_t)y * FCX + (Xa + 1 - FT / 2)] = -z.y;
-            } else {   // Xa == 0: column 0 becomes the last half-spectrum column
-                o[(size_t)y * FCX + FT / 2] = z.x;
-            }
+            s_blk[y * kLpPitch + cl] = v[P16(k)].x;          // conjugate: a' = Re, b' = -Im
+            s_blk[y * kLpPitch + cl + 1] = -v[P16(k)].y;
         }
+    }
+    __syncthreads();
+    if (c < nkeep) {
+#pragma unroll 8
+        for (int y = r; y < FT; y += RS) o[(size_t)y * FCX + c] = s_blk[y * kLpPitch + c];
     }
 }
 
@@ -1516,19 +1527,26 @@ k_lowpass_cols(const float* __restrict__ rowf, const float* __restrict__ ctf0, c
 
 int fused_tile_supported(int tile) { return tile == FT ? 1 : 0; }
 
-cudaError_t launch_lowpass512(const float* ctf0, const float2* tw, double bfactor, int nmic, const double* moments,
+cudaError_t launch_lp_axis(float* axis, double bfactor, cudaStream_t st)
+{
+    k_lp_axis<<<1, FT, 0, st>>>(axis, bfactor);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lowpass512(const float* ctf0, const float2* tw, const float* axis, int nmic, const double* moments,
                               float* rowf, float* out, int* lowpassed, cudaStream_t st)
 {
     if (nmic <= 0) return cudaSuccess;
     cudaError_t e = init_constants();
     if (e != cudaSuccess) return e;
-    k_lowpass_rows<<<dim3(FT / 2 / kLpWarps, nmic), kLpWarps * 32, 0, st>>>(ctf0, tw, bfactor, rowf);
+    k_lowpass_rows<<<dim3(FT / 2 / kLpWarps, nmic), kLpWarps * 32, 0, st>>>(ctf0, tw, axis, rowf);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const size_t sm = (size_t)FT * 33 * sizeof(float);
+    const size_t sm = (size_t)FT * kLpPitch * sizeof(float);
     if ((e = cudaFuncSetAttribute(k_lowpass_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
         cudaSuccess)
         return e;
-    k_lowpass_cols<<<dim3(9, nmic), kLpWarps * 32, sm, st>>>(rowf, ctf0, tw, bfactor, moments, out, lowpassed);
+    k_lowpass_cols<<<dim3(FT / 2 / kLpCols + 1, nmic), kLpWarps * 32, sm, st>>>(rowf, ctf0, tw, axis, moments, out,
+                                                                                lowpassed);
     return cudaGetLastError();
 }
 

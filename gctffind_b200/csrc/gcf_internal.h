@@ -249,17 +249,21 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
                          cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, const SoloLaunch* solo = nullptr);
 
 // gcf_post.cu
-void launch_bg_horizontal(const float* raw, int tile, int nmic, int log_spect, double* hsum,
-                          cudaStream_t st);
-void launch_bg_vertical(const float* raw, const double* hsum, int tile, int nmic, int log_spect,
-                        float* ctf, cudaStream_t st);
+// ctf = raw minus its box mean, and mom[m] = (mean, second moment) of ctf.
+// part: 2 x background_blocks(tile) doubles per spectrum; ticket: one per
+// spectrum, zero before the first launch and left zero.
+size_t background_blocks(int tile);
+cudaError_t launch_background(const float* raw, int tile, int nmic, int log_spect, float* ctf, double* part,
+                              unsigned* ticket, double* mom, cudaStream_t st);
 void launch_moments(const float* spect, int n, int nmic, double* out2, cudaStream_t st);
 // lowpass of CFindCtfBase::mLowpass around a batched R2C / C2R pair
 void launch_lp_full(const float* ctf0, int tile, int nmic, float* full, cudaStream_t st);
 // gcf_fused.cu: the whole lowpass of 512 x 512 spectra (ctf0 -> out, the
 // variance gate included) with the warp FFT; rowf: 512 x 512 floats per
-// spectrum of scratch; tw: exp(-2 pi i k / 512), k < 512.
-cudaError_t launch_lowpass512(const float* ctf0, const float2* tw, double bfactor, int nmic, const double* moments,
+// spectrum of scratch; tw: exp(-2 pi i k / 512), k < 512; axis: the filter's
+// 512 values of launch_lp_axis.
+cudaError_t launch_lp_axis(float* axis, double bfactor, cudaStream_t st);
+cudaError_t launch_lowpass512(const float* ctf0, const float2* tw, const float* axis, int nmic, const double* moments,
                               float* rowf, float* out, int* lowpassed, cudaStream_t st);
 void launch_lp_table(double* g, int tile, double bfactor, cudaStream_t st);
 void launch_lp_filter(float2* cmp, int tile, int nmic, const double* g, cudaStream_t st);

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "gcf_internal.h"
 
 namespace gcf {
@@ -47,106 +49,143 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh /* 32*NV *
     __syncthreads();
 }
 
-// Value of the background plane at relative position (u, R): the Hermitian
-// fold of GRmBackground2D::mGRemove (FindCTF/GRmBackground2D.cu:42-64).
-__device__ __forceinline__ float bg_val(const float* row, const float* mrow, int u, int half_x,
-                                        int tile)
-{
-    if (u >= half_x) u -= 2 * half_x;
-    (void)tile;
-    return (u >= 0) ? row[u] : mrow[-u];
-}
+// Background removal and the moments of its result (GRmBackground2D::mGRemove,
+// FindCTF/GRmBackground2D.cu:18-69): the box mean of sqrt(raw) (raw if
+// log_spect), squared again (log_spect: not), subtracted from raw outside the
+// DC mask (fR < 0.04).  The box is separable, its sums FP64.
+//
+// A block makes seg rows x strip columns of one spectrum: the values of its
+// rows and columns with the box's halo (rows modulo tile, columns folded at
+// the Hermitian edge, GRmBackground2D.cu:42-64) go to shared memory, threads
+// slide the vertical box down the columns, then the horizontal one along the
+// rows (one lane per row, odd pitches: no bank conflicts), and the block
+// writes its rows.  All intermediate sums stay in shared memory; the last
+// block of a spectrum adds the blocks' moments in block order.
+//
+// Bound: latency for few spectra; for many conversions to FP64 and shared-memory
+// reads (about 6 of each per output and direction) and the halo's square roots.
+// Two kernels with the horizontal sums in global memory and a third, one block
+// per spectrum, for the moments took 34.0 us for one spectrum of 512 x 257; this
+// kernel takes 13.9 us.  256 spectra: 517 us and 558 us, the price of one path.
+constexpr int kBgThreads = 576;   // at most; a whole number of column groups
 
-// Rows per block of the horizontal box sums (powers of two, so that the
-// 256 threads split evenly over the rows).
-__host__ __device__ constexpr int bg_rows_per_block(int tile)
+__global__ void __launch_bounds__(kBgThreads)
+k_background(const float* __restrict__ raw, int tile, int log_spect, int box, int seg, int strip,
+             float* __restrict__ ctf, double* __restrict__ part, unsigned* __restrict__ ticket,
+             double* __restrict__ mom)
 {
-    return tile <= 512 ? 8 : tile <= 1024 ? 4 : tile <= 2048 ? 2 : 1;
-}
-
-// Horizontal box sums of sqrt(raw) (or raw if log_spect) for every row and
-// every output column x in [0, cx).  A block holds bg_rows_per_block rows
-// and their mirror rows; each thread sums the box at the first column of
-// its run of consecutive columns and slides it over the rest (add the
-// entering, subtract the leaving value), in FP64.
-__global__ void __launch_bounds__(256) k_bg_horizontal(const float* __restrict__ raw, int tile, int log_spect,
-                                                       int box, double* __restrict__ hsum)
-{
-    extern __shared__ float sh[];
-    const int cx = tile / 2 + 1, half_x = cx - 1;
-    const int RB = bg_rows_per_block(tile), tpr = blockDim.x / RB;
-    const int r0 = blockIdx.x * RB, m = blockIdx.y;
-    const float* src = raw + (size_t)m * cx * tile;
-    for (int i = threadIdx.x; i < RB * cx; i += blockDim.x) {
-        const int rr = i / cx, x = i - rr * cx, R = r0 + rr;
-        if (R >= tile) continue;
-        const int mr = (tile - R) % tile;   // half_y - (R - half_y) modulo tile
-        float a = src[(size_t)R * cx + x], b = src[(size_t)mr * cx + x];
-        sh[rr * 2 * cx + x] = log_spect ? a : sqrtf(a);
-        sh[rr * 2 * cx + cx + x] = log_spect ? b : sqrtf(b);
+    extern __shared__ double s_bg[];
+    __shared__ double s_red[64];
+    const int cx = tile / 2 + 1, half_x = cx - 1, hb = box / 2, m = blockIdx.y;
+    const int strips = (cx + strip - 1) / strip;
+    const int x0 = (int)(blockIdx.x % strips) * strip, w = min(strip, cx - x0), e = w + 2 * hb;
+    const int y0 = (int)(blockIdx.x / strips) * seg, h = min(seg, tile - y0), rows = h + 2 * hb;
+    const int pe = (strip + 2 * hb) | 1, ps = strip | 1;
+    double* V = s_bg;                                        // [seg][pe] vertical sums
+    float* A = reinterpret_cast<float*>(s_bg + seg * pe);    // [seg + 2 hb][pe] values
+    double* S = s_bg + seg * pe;                             // [seg][ps] box sums, over A
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int NW = blockDim.x >> 5;
+    const size_t base = (size_t)m * cx * tile;
+    const float* src = raw + base;
+    // a thread keeps one column: its fold is decided once
+    const int ew = (strip + 2 * hb + 31) & ~31, G = blockDim.x / ew, g = tid / ew, c0 = tid - g * ew;
+    if (c0 < e && g < G) {
+        int u = x0 - hb + c0;
+        if (u >= half_x) u -= 2 * half_x;
+        const bool fold = u < 0;
+        const float* col = src + (fold ? -u : u);
+        float* a = A + c0;
+#pragma unroll 4
+        for (int r = g; r < rows; r += G) {
+            int R = y0 - hb + r;
+            if (R < 0) R += tile;
+            else if (R >= tile) R -= tile;
+            if (fold && R) R = tile - R;   // half_y - (R - half_y) modulo tile
+            const float v = __ldg(col + (size_t)R * cx);
+            a[r * pe] = log_spect ? v : sqrtf(v);
+        }
     }
     __syncthreads();
-    const int rr = threadIdx.x / tpr, t = threadIdx.x - rr * tpr, R = r0 + rr;
-    if (rr >= RB || R >= tile) return;
-    const float* row = sh + rr * 2 * cx;
-    const float* mrow = row + cx;
-    const int seg = (cx + tpr - 1) / tpr;
-    const int x0 = t * seg, x1 = min(cx, x0 + seg);
-    if (x0 >= x1) return;
-    const int hb = box / 2;
-    double* out = hsum + ((size_t)m * tile + R) * cx;
-    double sum = 0.0;
-    for (int j = -hb; j <= hb; ++j) sum += (double)bg_val(row, mrow, x0 + j, half_x, tile);
-    out[x0] = sum;
-    for (int x = x0 + 1; x < x1; ++x) {
-        sum += (double)bg_val(row, mrow, x + hb, half_x, tile) - (double)bg_val(row, mrow, x - 1 - hb, half_x, tile);
-        out[x] = sum;
-    }
-}
-
-// Vertical box sums, DC mask (fR < 0.04) and subtraction
-// (FindCTF/GRmBackground2D.cu:18-31, :67-69).  A block covers kBgSegY rows
-// of every column; each thread slides the vertical box down its column (one
-// column per thread up to tile 1024: the block has cx threads rounded up to
-// whole warps, at most kBgVertThreads).
-constexpr int kBgSegY = 16;
-constexpr int kBgVertThreads = 544;
-__global__ void k_bg_vertical(const float* __restrict__ raw, const double* __restrict__ hsum,
-                                                     int tile, int log_spect, int box, float* __restrict__ ctf)
-{
-    const int cx = tile / 2 + 1, cy = tile;
-    const int m = blockIdx.y;
-    const int y0 = blockIdx.x * kBgSegY, y1 = min(cy, y0 + kBgSegY);
-    const size_t base = (size_t)m * cx * cy;
-    const int hb = box / 2;
-    const double norm = (double)box * (double)box;
-    for (int x = threadIdx.x; x < cx; x += blockDim.x) {
+    if (c0 < e && g < G) {   // G runs of rows per column
+        const int c = c0, ya = h * g / G, yb = h * (g + 1) / G;
         double sum = 0.0;
-        for (int k = -hb; k <= hb; ++k) {
-            int yy = y0 + k;
-            if (yy < 0) yy += cy;
-            else if (yy >= cy) yy -= cy;
-            sum += hsum[base + (size_t)yy * cx + x];
+#pragma unroll 4
+        for (int k = 0; k <= 2 * hb; ++k) sum += (double)A[(ya + k) * pe + c];
+        if (ya < yb) V[ya * pe + c] = sum;
+#pragma unroll 4
+        for (int y = ya + 1; y < yb; ++y) {
+            sum += (double)A[(y + 2 * hb) * pe + c] - (double)A[(y - 1) * pe + c];
+            V[y * pe + c] = sum;
         }
-        for (int y = y0; y < y1; ++y) {
-            if (y > y0) {
-                int yin = y + hb, yout = y - 1 - hb;
-                if (yin >= cy) yin -= cy;
-                if (yout < 0) yout += cy;
-                sum += hsum[base + (size_t)yin * cx + x] - hsum[base + (size_t)yout * cx + x];
+    }
+    __syncthreads();
+    {
+        const int xa = w * warp / NW, xb = w * (warp + 1) / NW;   // this warp's columns
+        for (int y = lane; y < h && xa < xb; y += 32) {
+            const double* v = V + y * pe;
+            double sum = 0.0;
+#pragma unroll 4
+            for (int k = 0; k <= 2 * hb; ++k) sum += v[xa + k];
+            S[y * ps + xa] = sum;
+#pragma unroll 4
+            for (int x = xa + 1; x < xb; ++x) {
+                sum += v[x + 2 * hb] - v[x - 1];
+                S[y * ps + x] = sum;
             }
-            const int i = y * cx + x;
-            const int yr = y - cy / 2;
-            float fr = x * 0.5f / (cx - 1);
-            fr = sqrtf(fr * fr + yr * yr / (float)(cy * cy));
-            if ((double)fr < 0.04) {
-                ctf[base + i] = 0.0f;
-                continue;
+        }
+    }
+    __syncthreads();
+    const double norm = (double)box * (double)box, inv = 1.0 / norm;
+    double mv[2] = {0.0, 0.0};
+    for (int r = warp; r < h; r += NW) {
+        const int y = y0 + r, yr = y - tile / 2;
+#pragma unroll 4
+        for (int c = lane; c < w; c += 32) {
+            const int x = x0 + c;
+            const size_t i = base + (size_t)y * cx + x;
+            bool masked = false;
+            if (12 * x < cx) {   // beyond, x * 0.5 / (cx - 1) alone is above 0.04
+                float fr = x * 0.5f / (cx - 1);
+                fr = sqrtf(fr * fr + yr * yr / (float)(tile * tile));
+                masked = (double)fr < 0.04;
             }
-            double b = sum / norm;
+            // sum / norm: the reciprocal's product with its residual added back
+            // (Markstein); a division of its own costs 90 us at 256 spectra
+            const double sum = S[r * ps + c];
+            double b = sum * inv;
+            b = __fma_rn(__fma_rn(-b, norm, sum), inv, b);
             if (!log_spect) b *= b;
-            ctf[base + i] = (float)((double)raw[base + i] - b);
+            const float v = masked ? 0.0f : (float)((double)__ldg(raw + i) - b);
+            ctf[i] = v;
+            mv[0] += (double)v;
+            mv[1] += (double)v * (double)v;
         }
+    }
+    block_sum<2>(mv, s_red);
+    if (warp != 0) return;
+    const int nb = gridDim.x;
+    double* p = part + 2 * (size_t)m * nb;
+    int last = 0;
+    if (lane == 0) {
+        p[2 * blockIdx.x] = mv[0];
+        p[2 * blockIdx.x + 1] = mv[1];
+        __threadfence();
+        last = atomicInc(ticket + m, nb - 1) == (unsigned)(nb - 1);   // wraps to zero for the next launch
+        __threadfence();
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    mv[0] = mv[1] = 0.0;
+    for (int k = lane; k < nb; k += 32) {
+        mv[0] += __ldcg(p + 2 * k);
+        mv[1] += __ldcg(p + 2 * k + 1);
+    }
+    mv[0] = warp_sum(mv[0]);
+    mv[1] = warp_sum(mv[1]);
+    if (lane == 0) {
+        const int n = cx * tile;
+        mom[2 * m] = mv[0] / n;
+        mom[2 * m + 1] = mv[1] / n;
     }
 }
 
@@ -445,32 +484,59 @@ __global__ void k_shell_cc(int tile, const double* __restrict__ ring_sums, float
 
 }  // namespace
 
-void launch_bg_horizontal(const float* raw, int tile, int nmic, int log_spect, double* hsum,
-                          cudaStream_t st)
+namespace {
+
+// Rows and columns of a background block.
+struct BgShape {
+    int box, seg, strip;
+    size_t smem;
+    int blocks(int tile) const { return ((tile / 2 + strip) / strip) * ((tile + seg - 1) / seg); }
+};
+
+BgShape bg_shape(int tile, int nmic)
 {
     // box of GRmBackground2D::mGRemove (FindCTF/GRmBackground2D.cu:33-36), fMinFreq = 1/15
-    float fmin = 1.0f / 15.0f;
+    const float fmin = 1.0f / 15.0f;
     int box = (int)(fmin * tile);
     if (box > (0.3f * tile)) box = (int)(0.3f * tile);
     box = box / 2 * 2 + 1;
     if (box < 7) box = 7;
-    int cx = tile / 2 + 1, rb = bg_rows_per_block(tile);
-    dim3 grid((tile + rb - 1) / rb, nmic);
-    k_bg_horizontal<<<grid, 256, 2 * rb * cx * sizeof(float), st>>>(raw, tile, log_spect, box, hsum);
+    BgShape b{box, 8, 0, 0};
+    const int cx = tile / 2 + 1, hb = box / 2;
+    // strips of at most 160 columns, narrower until two blocks fit an SM
+    auto fit = [&](int seg) {
+        b.seg = seg;
+        for (int n = (cx + 159) / 160;; ++n) {
+            b.strip = (cx + n - 1) / n;
+            const size_t pe = (size_t)(b.strip + 2 * hb) | 1, ps = (size_t)b.strip | 1;
+            b.smem = (size_t)seg * pe * 8 + std::max((size_t)(seg + 2 * hb) * pe * 4, (size_t)seg * ps * 8);
+            if (b.smem <= 110 * 1024 || b.strip <= 8) break;
+        }
+    };
+    // 8 rows while the chip takes all blocks at once (two per SM), else 32,
+    // which halve the halo's share: 512 x 257 spectra, 17.8 (8 rows) and 23.8 us
+    // (32) for one, 21.1 and 24.5 for two, 32.9 and 25.2 for four, 1427 and 560
+    // for 256, launch included.
+    fit(8);
+    if ((long long)b.blocks(tile) * nmic > 2 * 148) fit(32);
+    return b;
 }
 
-void launch_bg_vertical(const float* raw, const double* hsum, int tile, int nmic, int log_spect,
-                        float* ctf, cudaStream_t st)
+}  // namespace
+
+size_t background_blocks(int tile) { return bg_shape(tile, 1).blocks(tile); }
+
+cudaError_t launch_background(const float* raw, int tile, int nmic, int log_spect, float* ctf, double* part,
+                              unsigned* ticket, double* mom, cudaStream_t st)
 {
-    float fmin = 1.0f / 15.0f;
-    int box = (int)(fmin * tile);
-    if (box > (0.3f * tile)) box = (int)(0.3f * tile);
-    box = box / 2 * 2 + 1;
-    if (box < 7) box = 7;
-    int cx = tile / 2 + 1;
-    int th = std::min(kBgVertThreads, ((cx + 31) / 32) * 32);
-    dim3 grid((tile + kBgSegY - 1) / kBgSegY, nmic);
-    k_bg_vertical<<<grid, th, 0, st>>>(raw, hsum, tile, log_spect, box, ctf);
+    const BgShape b = bg_shape(tile, nmic);
+    const int ew = (b.strip + 2 * (b.box / 2) + 31) & ~31;
+    const int threads = ew * std::max(1, kBgThreads / ew);
+    cudaError_t e = cudaFuncSetAttribute(k_background, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
+    if (e != cudaSuccess) return e;
+    k_background<<<dim3(b.blocks(tile), nmic), threads, b.smem, st>>>(raw, tile, log_spect, b.box, b.seg, b.strip,
+                                                                         ctf, part, ticket, mom);
+    return cudaGetLastError();
 }
 
 void launch_moments(const float* spect, int n, int nmic, double* out2, cudaStream_t st)
