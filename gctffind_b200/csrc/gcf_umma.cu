@@ -628,6 +628,12 @@ k_umma_gemm_pair(const __grid_constant__ CUtensorMap ta, const __grid_constant__
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
     }
+    // The pair's allocation takes columns on both SMs: the other CTA has to be
+    // running.  Without this barrier a pair that started while another launch
+    // was leaving its SMs could wait in the allocation for good (two streams of
+    // these products: about one call in a few hundred).
+    __syncwarp();
+    cluster_sync_all();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_taddr)),
                      "r"(2 * BN)
