@@ -1671,6 +1671,27 @@ struct RescaleLanes {
         }
         return GCF_OK;
     }
+    // The lanes' scratch for a whole call at once: an uneven batch that grew it
+    // image by image freed and allocated it up to 37 times on its first call.
+    gcf_status reserve(const int* ws, const int* hs, const float* pxs, int n)
+    {
+        size_t bf[2] = {}, f32[2] = {};
+        for (int i = 0, u = 0; i < n && ctx->rescale_impl == GCF_RESCALE_GEMM; ++i) {
+            int nw, nh;
+            float pn;
+            gcf_rescale_dims(ws[i], hs[i], pxs[i], &nw, &nh, &pn);
+            if (1.2f / pxs[i] <= 1 || !rescale_gemm_supported(ws[i], hs[i], nw, nh)) continue;
+            const RescaleGemmLayout L = rescale_gemm_layout(ws[i], hs[i], nw, nh);
+            bf[u & 1] = std::max(bf[u & 1], (size_t)L.bf16_elems);
+            f32[u & 1] = std::max(f32[u & 1], (size_t)L.f32_elems);
+            ++u;
+        }
+        for (int k = 0; k < 2; ++k) {
+            if (bf[k]) CK(ctx->rsg_bf[k].ensure(bf[k]));
+            if (f32[k]) CK(ctx->rsg_f[k].ensure(f32[k]));
+        }
+        return GCF_OK;
+    }
     // The compute stream continues after both lanes.
     gcf_status join()
     {
@@ -1826,6 +1847,7 @@ gcf_status prepare_images(gcf_ctx* ctx, const float* const* images, const int* w
     CK(record_timing(ctx->ev[2], ctx->st));
     size_t roff = 0, roff_new = 0;
     RescaleLanes lanes(ctx);
+    CKS(lanes.reserve(ws, hs, pxs, n));
     for (int c = 0; c < nchunks; ++c) {
         int i0 = c * kChunk, i1 = std::min(n, i0 + kChunk);
         std::vector<const float*> dimg(i1 - i0);
