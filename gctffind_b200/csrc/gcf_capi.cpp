@@ -17,6 +17,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <initializer_list>
 #include <vector>
 
 #include "gcf_internal.h"
@@ -340,9 +341,13 @@ namespace {
 // copy stream, which would hold the compute stream until every image had
 // landed).  Outside a capture, an arena that has grown past 64 MB is
 // recycled once the context's streams are idle.
-cudaError_t h2d(gcf_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st)
+struct HostPiece {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+cudaError_t h2d(gcf_ctx* ctx, std::initializer_list<HostPiece> pieces, cudaStream_t st)
 {
-    if (bytes == 0) return cudaSuccess;
     if (!ctx->capturing) {
         size_t used = 0;
         for (const HostArena::Block& b : ctx->arena.blocks) used += b.used;
@@ -355,10 +360,23 @@ cudaError_t h2d(gcf_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStre
             ctx->arena.reset();
         }
     }
-    void* h = ctx->arena.put(src, bytes);
-    if (!h) return cudaErrorMemoryAllocation;
+    HostPieces p;
+    for (const HostPiece& q : pieces) {
+        if (q.bytes == 0) continue;
+        if (p.n == HostPieces::kMax) return cudaErrorInvalidValue;
+        const void* h = ctx->arena.put(q.src, q.bytes);
+        if (!h) return cudaErrorMemoryAllocation;
+        p.dst[p.n] = static_cast<unsigned char*>(q.dst);
+        p.src[p.n] = static_cast<const unsigned char*>(h);
+        p.bytes[p.n++] = q.bytes;
+    }
+    if (p.n == 0) return cudaSuccess;
     ctx->launches += 1;
-    return launch_copy_from_host(dst, h, bytes, st);
+    return launch_copy_from_host(p, st);
+}
+cudaError_t h2d(gcf_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    return h2d(ctx, {{dst, src, bytes}}, st);
 }
 
 gcf_status fail(gcf_ctx* c, gcf_status s, const char* what)
@@ -586,12 +604,14 @@ gcf_status get_band(gcf_ctx* ctx, const gcf_optics& op, float px_n, int* slot)
     }
     // On the compute stream, so the kernels that read the band are ordered
     // after the copies (a pageable source is staged before the call returns).
-    CK(h2d(ctx, b->idx.p, idx.data(), n * sizeof(int), ctx->st));
-    CK(h2d(ctx, b->a.p, va.data(), n * sizeof(float), ctx->st));
-    CK(h2d(ctx, b->d.p, vd.data(), n * sizeof(float), ctx->st));
-    CK(h2d(ctx, b->env.p, ve.data(), n * sizeof(float), ctx->st));
-    CK(h2d(ctx, b->c2t.p, vc.data(), n * sizeof(float), ctx->st));
-    CK(h2d(ctx, b->s2t.p, vs.data(), n * sizeof(float), ctx->st));
+    CK(h2d(ctx,
+           {{b->idx.p, idx.data(), n * sizeof(int)},
+            {b->a.p, va.data(), n * sizeof(float)},
+            {b->d.p, vd.data(), n * sizeof(float)},
+            {b->env.p, ve.data(), n * sizeof(float)},
+            {b->c2t.p, vc.data(), n * sizeof(float)},
+            {b->s2t.p, vs.data(), n * sizeof(float)}},
+           ctx->st));
     b->dev.n = b->n;
     b->dev.cx = cx;
     b->dev.cy = cy;
@@ -825,7 +845,6 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
         bptr[i] = ctx->f_bsum.p + boff[i];
         d[i].bsum = bptr[i];
     }
-    CK(h2d(ctx, ctx->f_bsum_ptr.p, bptr.data(), nm * sizeof(double*), ctx->st));
     CK(ctx->f_desc.ensure(nm));
     CK(ctx->f_items.ensure(ni));
     CK(ctx->f_first.ensure(nm + 1));
@@ -833,11 +852,14 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
     CK(ctx->f_inv.ensure(nm));
     CK(ctx->f_partial.ensure((size_t)ni * cx * T));
     CK(ctx->f_next.ensure(nm));
-    CK(h2d(ctx, ctx->f_desc.p, d.data(), nm * sizeof(FusedImageDesc), ctx->st));
-    CK(h2d(ctx, ctx->f_items.p, items.data(), ni * sizeof(int4), ctx->st));
-    CK(h2d(ctx, ctx->f_first.p, first.data(), (nm + 1) * sizeof(int), ctx->st));
-    CK(h2d(ctx, ctx->f_group.p, group.data(), nm * sizeof(int), ctx->st));
-    CK(h2d(ctx, ctx->f_inv.p, inv.data(), nm * sizeof(float), ctx->st));
+    CK(h2d(ctx,
+           {{ctx->f_bsum_ptr.p, bptr.data(), nm * sizeof(double*)},
+            {ctx->f_desc.p, d.data(), nm * sizeof(FusedImageDesc)},
+            {ctx->f_items.p, items.data(), ni * sizeof(int4)},
+            {ctx->f_first.p, first.data(), (nm + 1) * sizeof(int)},
+            {ctx->f_group.p, group.data(), nm * sizeof(int)},
+            {ctx->f_inv.p, inv.data(), nm * sizeof(float)}},
+           ctx->st));
     return GCF_OK;
 }
 
@@ -1163,8 +1185,8 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     const int k0 = steps & 1;
     SearchJob* const jobs0 = ctx->jobs.p + (size_t)k0 * nj;
     CK(cudaMemsetAsync(ctx->arrive.p, 0, (size_t)nj * (1 + kMaxCandBlocks) * sizeof(int), ctx->st));
-    CK(h2d(ctx, jobs0, jh.data(), nj * sizeof(SearchJob), ctx->st));
-    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int2), ctx->st));
+    CK(h2d(ctx, {{jobs0, jh.data(), nj * sizeof(SearchJob)}, {ctx->spec_off.p, soff.data(), nj * sizeof(int2)}},
+           ctx->st));
     launch_band_gather(ctx->ctf.p, (int)cmp_n, jobs0, ctx->d_bands.p, ctx->spec_off.p, nj,
                        ctx->band_spec.p, ctx->sum_ss.p, ctx->st);
     CKL();
@@ -1345,8 +1367,8 @@ gcf_status run_fast_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, con
     CK(ctx->cc_res.ensure((size_t)nj * cx));
     CK(ctx->d_res.ensure(nj));
     CK(cudaMemsetAsync(ctx->arrive.p, 0, (size_t)nj * (1 + kMaxCandBlocks) * sizeof(int), ctx->st));
-    CK(h2d(ctx, ctx->jobs.p, jh.data(), nj * sizeof(SearchJob), ctx->st));
-    CK(h2d(ctx, ctx->spec_off.p, soff.data(), nj * sizeof(int2), ctx->st));
+    CK(h2d(ctx, {{ctx->jobs.p, jh.data(), nj * sizeof(SearchJob)}, {ctx->spec_off.p, soff.data(), nj * sizeof(int2)}},
+           ctx->st));
     CK(record_timing(ctx->ev[5], ctx->st));
     launch_band_gather(ctx->ctf.p, (int)cmp_n, ctx->jobs.p, ctx->d_bands.p, ctx->spec_off.p, nj, ctx->band_spec.p,
                        ctx->sum_ss.p, ctx->st);
@@ -1936,9 +1958,11 @@ gcf_status full_spectra(gcf_ctx* ctx, const std::vector<int>& mics,
     CK(ctx->mic_of.ensure(k));
     CK(ctx->d_res.ensure(std::max<size_t>(k, ctx->d_res.n)));
     CK(ctx->full.ensure((size_t)k * T * T));
-    CK(h2d(ctx, ctx->d_optics.p, o.data(), k * sizeof(PixOptics), ctx->st));
-    CK(h2d(ctx, ctx->mic_of.p, mics.data(), k * sizeof(int), ctx->st));
-    CK(h2d(ctx, ctx->d_res.p, res.data(), k * sizeof(gcf_result), ctx->st));
+    CK(h2d(ctx,
+           {{ctx->d_optics.p, o.data(), k * sizeof(PixOptics)},
+            {ctx->mic_of.p, mics.data(), k * sizeof(int)},
+            {ctx->d_res.p, res.data(), k * sizeof(gcf_result)}},
+           ctx->st));
     launch_full_spectrum(ctx->ctf.p, T, k, ctx->mic_of.p, ctx->d_res.p, ctx->d_optics.p,
                          ctx->moments2.p, 0.0f, ctx->full.p, ctx->st);
     CKL();
@@ -2388,8 +2412,8 @@ static gcf_status remove_bg(gcf_ctx* ctx, float* spec, size_t spec_n, int n_or_t
     if (!on_device) {
         CK(ctx->bg_spec.ensure(spec_n));
         CK(ctx->bg_curve.ensure(bg_n));
-        CK(h2d(ctx, ctx->bg_spec.p, spec, spec_n * sizeof(float), ctx->st));
-        CK(h2d(ctx, ctx->bg_curve.p, bg, bg_n * sizeof(float), ctx->st));
+        CK(h2d(ctx, {{ctx->bg_spec.p, spec, spec_n * sizeof(float)}, {ctx->bg_curve.p, bg, bg_n * sizeof(float)}},
+               ctx->st));
         d_spec = ctx->bg_spec.p;
         d_bg = ctx->bg_curve.p;
     }

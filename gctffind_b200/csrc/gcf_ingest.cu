@@ -88,14 +88,19 @@ __global__ void k_mrc_to_float(const unsigned char* __restrict__ raw, int mode, 
 
 namespace {
 
-// dst[0, bytes) = src[0, bytes) with src in mapped page-locked host memory:
-// 16-byte words where both sides allow, bytes at the ends.
-__global__ void k_copy_from_host(unsigned char* __restrict__ dst, const unsigned char* __restrict__ src,
-                                 size_t bytes, int vec)
+// Piece blockIdx.y: dst[0, bytes) = src[0, bytes) with src in mapped
+// page-locked host memory: 16-byte words where both sides allow, bytes at the
+// ends.  Bound: one round trip to the host per launch, about 3 us and as much
+// again between launches, so the tables of a call go in one launch (the six of
+// a tile plan and the two of a search were a launch each).
+__global__ void k_copy_from_host(HostPieces p)
 {
+    unsigned char* __restrict__ dst = p.dst[blockIdx.y];
+    const unsigned char* __restrict__ src = p.src[blockIdx.y];
+    const size_t bytes = p.bytes[blockIdx.y];
     const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     size_t done = 0;
-    if (vec) {
+    if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0) {
         const size_t words = bytes / 16;
         for (size_t i = tid; i < words; i += nth)
             reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
@@ -106,13 +111,13 @@ __global__ void k_copy_from_host(unsigned char* __restrict__ dst, const unsigned
 
 }  // namespace
 
-cudaError_t launch_copy_from_host(void* dst, const void* src_mapped, size_t bytes, cudaStream_t st)
+cudaError_t launch_copy_from_host(const HostPieces& p, cudaStream_t st)
 {
-    if (bytes == 0) return cudaSuccess;
-    const int vec = (((uintptr_t)dst | (uintptr_t)src_mapped) % 16) == 0;
-    const int blocks = (int)std::min<size_t>((bytes / 16 + 255) / 256 + 1, 148);
-    k_copy_from_host<<<blocks, 256, 0, st>>>(static_cast<unsigned char*>(dst),
-                                             static_cast<const unsigned char*>(src_mapped), bytes, vec);
+    size_t most = 0;
+    for (int k = 0; k < p.n; ++k) most = std::max(most, p.bytes[k]);
+    if (most == 0) return cudaSuccess;
+    const int blocks = (int)std::min<size_t>((most / 16 + 255) / 256 + 1, 148);
+    k_copy_from_host<<<dim3(blocks, p.n), 256, 0, st>>>(p);
     return cudaGetLastError();
 }
 

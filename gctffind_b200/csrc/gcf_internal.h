@@ -68,7 +68,14 @@ cudaError_t launch_mrc_to_float(const void* raw, int mode, int swap, size_t npx,
 // (src_mapped: its device-side address).  Small uploads take this route
 // instead of a copy-engine transfer, so they never queue behind the bulk
 // image uploads on the copy engines.
-cudaError_t launch_copy_from_host(void* dst, const void* src_mapped, size_t bytes, cudaStream_t st);
+struct HostPieces {
+    static constexpr int kMax = 8;
+    int n = 0;
+    unsigned char* dst[kMax];
+    const unsigned char* src[kMax];   // mapped page-locked memory
+    size_t bytes[kMax];
+};
+cudaError_t launch_copy_from_host(const HostPieces& p, cudaStream_t st);
 
 constexpr int kMaxCand = 2624;        // >= 51 * 51 astigmatism grid
 constexpr int kEvalThreads = 256;     // threads of the candidate kernel
