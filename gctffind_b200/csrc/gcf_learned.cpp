@@ -270,8 +270,14 @@ static cudaError_t layer_dx(NnNet* n, int li, const __nv_bfloat16* dz, long long
     g.D = dx;
     g.ldd = l.in;
     g.err = n->err.p;
-    const int bn = l.in <= 32 ? 32 : (l.in <= 64 ? 64 : (l.in <= 128 ? 128 : 256));
-    return launch_umma_gemm(dz, ldz, n->wt.p + n->wt_off[li], l.ldt, g, bn, bn == 256 ? 3 : 4, 0, st);
+    // K is one to four slices and the FP32 rows are many: writing them bounds
+    // the product, so what counts is how many CTAs share an SM.  Tiles of 64
+    // columns with two stages let four in: 262144 x 144 x 32 61.9 us (tiles of
+    // 256, one CTA per SM, 146.9; the persistent kernel 100 to 145),
+    // 65536 x 288 x 32 27.0 us (71.5), 16384 x 288 x 32 10.0 us (21.2).  Few
+    // rows are latency: 256 x 256 x 128 4.5 us (9.6), 256 x 2304 x 256 5.6 us
+    // (10.6).
+    return launch_umma_gemm(dz, ldz, n->wt.p + n->wt_off[li], l.ldt, g, 64, 2, 0, st);
 }
 
 static cudaError_t layer_dw(NnNet* n, int li, const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* in,
