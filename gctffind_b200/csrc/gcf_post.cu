@@ -66,10 +66,11 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh /* 32*NV *
 // reads (about 6 of each per output and direction) and the halo's square roots.
 // Two kernels with the horizontal sums in global memory and a third, one block
 // per spectrum, for the moments took 34.0 us for one spectrum of 512 x 257; this
-// kernel takes 13.9 us.  256 spectra: 517 us and 558 us, the price of one path.
-constexpr int kBgThreads = 576;   // at most; a whole number of column groups
+// kernel takes 12.7 us; 256 spectra 517 us, now 458.  One spectrum of tile 1024:
+// 62.6 -> 29.2 us, of tile 2048: 193 -> 166 us.
+constexpr int kBgThreads = 640;   // at most, two blocks per SM; a whole number of column groups
 
-__global__ void __launch_bounds__(kBgThreads)
+__global__ void __maxnreg__(48)   // two blocks of 640 threads per SM
 k_background(const float* __restrict__ raw, int tile, int log_spect, int box, int seg, int strip,
              float* __restrict__ ctf, double* __restrict__ part, unsigned* __restrict__ ticket,
              double* __restrict__ mom)
@@ -121,8 +122,10 @@ k_background(const float* __restrict__ raw, int tile, int log_spect, int box, in
     }
     __syncthreads();
     {
-        const int xa = w * warp / NW, xb = w * (warp + 1) / NW;   // this warp's columns
-        for (int y = lane; y < h && xa < xb; y += 32) {
+        // a warp takes 32 rows and a run of columns
+        const int RB = (seg + 31) / 32, CG = max(NW / RB, 1);
+        const int xa = w * (warp / RB) / CG, xb = w * (warp / RB + 1) / CG;
+        for (int y = 32 * (warp % RB) + lane; y < h && xa < xb && warp / RB < CG; y += 32 * RB) {
             const double* v = V + y * pe;
             double sum = 0.0;
 #pragma unroll 4
@@ -486,6 +489,9 @@ __global__ void k_shell_cc(int tile, const double* __restrict__ ring_sums, float
 
 namespace {
 
+// Shared memory of a background block at two blocks, or one, per SM.
+constexpr size_t kTwoPerSM = 110 * 1024, kOnePerSM = 200 * 1024;
+
 // Rows and columns of a background block.
 struct BgShape {
     int box, seg, strip;
@@ -503,22 +509,31 @@ BgShape bg_shape(int tile, int nmic)
     if (box < 7) box = 7;
     BgShape b{box, 8, 0, 0};
     const int cx = tile / 2 + 1, hb = box / 2;
-    // strips of at most 160 columns, narrower until two blocks fit an SM
-    auto fit = [&](int seg) {
+    // strips of at most 160 columns, narrower until a block's shared memory fits
+    auto fit = [&](int seg, size_t limit) {
         b.seg = seg;
         for (int n = (cx + 159) / 160;; ++n) {
             b.strip = (cx + n - 1) / n;
             const size_t pe = (size_t)(b.strip + 2 * hb) | 1, ps = (size_t)b.strip | 1;
             b.smem = (size_t)seg * pe * 8 + std::max((size_t)(seg + 2 * hb) * pe * 4, (size_t)seg * ps * 8);
-            if (b.smem <= 110 * 1024 || b.strip <= 8) break;
+            if (b.smem <= limit || b.strip <= 8) break;
         }
     };
-    // 8 rows while the chip takes all blocks at once (two per SM), else 32,
-    // which halve the halo's share: 512 x 257 spectra, 17.8 (8 rows) and 23.8 us
-    // (32) for one, 21.1 and 24.5 for two, 32.9 and 25.2 for four, 1427 and 560
-    // for 256, launch included.
-    fit(8);
-    if ((long long)b.blocks(tile) * nmic > 2 * 148) fit(32);
+    // 8 rows while the chip takes all blocks at once (two per SM), then 32, then
+    // 64, which load less halo per output: 512 x 257 spectra, 17.8 (8 rows) and
+    // 23.8 us (32) for one, 21.1 and 24.5 for two, 32.9 and 24.7 (64 rows: 27.1)
+    // for four, 43.5 and 31.8 us (32 and 64) for 12, 566 and 473 us for 256,
+    // launch included.  Tiles whose box is wide leave 64 rows too narrow a strip,
+    // and from 2048 on 32 rows as well unless a block has an SM to itself.
+    auto one_wave = [&] { return (long long)b.blocks(tile) * nmic <= 2 * 148; };
+    fit(8, kTwoPerSM);
+    if (!one_wave()) fit(32, kTwoPerSM);
+    if (b.strip < 48 && b.strip < cx) fit(32, kOnePerSM);
+    if (!one_wave()) {
+        const BgShape rows32 = b;
+        fit(64, kTwoPerSM);
+        if (b.strip < 64 && b.strip < cx) b = rows32;
+    }
     return b;
 }
 
@@ -531,7 +546,7 @@ cudaError_t launch_background(const float* raw, int tile, int nmic, int log_spec
 {
     const BgShape b = bg_shape(tile, nmic);
     const int ew = (b.strip + 2 * (b.box / 2) + 31) & ~31;
-    const int threads = ew * std::max(1, kBgThreads / ew);
+    const int threads = ew * std::max(1, (b.smem > kTwoPerSM ? 1024 : kBgThreads) / ew);
     cudaError_t e = cudaFuncSetAttribute(k_background, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
     if (e != cudaSuccess) return e;
     k_background<<<dim3(b.blocks(tile), nmic), threads, b.smem, st>>>(raw, tile, log_spect, b.box, b.seg, b.strip,

@@ -1,14 +1,14 @@
 """Background removal over tile sizes, edges of its blocks and both spectrum
 kinds.
 
-A block covers 8 rows, or 32 when the call has more blocks than the chip takes
-at once, and a strip of columns (one strip up to tile 256, more above), so the
-tile sizes below have partial strips and the row and column folds in different
-blocks; 16 is the smallest tile and 90 leaves partial blocks of rows.  A faint image keeps the variance of the result below 1, so
-that the half spectrum comes back without the lowpass.  The reference takes
-the same float32 square roots and FP64 box sums: what remains is the final
-rounding to float32 (6e-8 relative) and FP64 sums in another order, which
-leave at most 1e-12 of the local background.
+A block covers 8 rows, or 32 or 64 when the call has more blocks than the chip
+takes at once, and a strip of columns (one strip up to tile 256, more above), so
+the tile sizes below have partial strips and the row and column folds in different
+blocks; 16 is the smallest tile and 90 leaves partial blocks of rows.  A faint
+image keeps the variance of the result below 1, so that the half spectrum comes
+back without the lowpass.  The reference takes the same float32 square roots and
+FP64 box sums: what remains is the final rounding to float32 (6e-8 relative) and
+FP64 sums in another order, which leave at most 1e-12 of the local background.
 """
 import numpy as np
 import pytest
@@ -61,7 +61,7 @@ def test_background_removed(gpu_lib, tile, log):
 
 @pytest.mark.parametrize("tile,count", [(90, 46), (512, 9), (1024, 5), (2048, 2)])
 def test_blocks_of_32_rows_match_blocks_of_8(gpu_lib, tile, count):
-    """Spectra made together (blocks of 32 rows) against the same spectra made
+    """Spectra made together (blocks of 32 or 64 rows) against the same spectra made
     one by one, by the per-micrograph cuFFT path, whose raw spectra do not
     depend on the company.  The right half of a full spectrum is the half
     spectrum without its last column."""
