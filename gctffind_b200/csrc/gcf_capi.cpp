@@ -1678,6 +1678,13 @@ struct RescaleLanes {
         const void* at = nullptr;
     } maps[2];
     explicit RescaleLanes(gcf_ctx* c) : ctx(c) {}
+    RescaleLanes(const RescaleLanes&) = delete;
+    RescaleLanes& operator=(const RescaleLanes&) = delete;
+    // A call that fails between next() and join() (an image too small for a
+    // tile, no memory) joins too: the second lane may still be writing the
+    // rescaled images and its scratch, which the next call's work on the
+    // compute stream uses again.
+    ~RescaleLanes() { join(); }
     // The lane of the next image; the first use of the second lane orders it
     // after everything on the compute stream.
     gcf_status next(int* lane, cudaStream_t* st)
