@@ -1213,7 +1213,7 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (want + per_y - 1) / per_y));
     for (int k = 0; k < steps; ++k) {
         int cb = (k == 0) ? 1 : (k == 1 && any_grid) ? (kMaxCand / kEvalCB + 3) / 4 : line_cb;
-        CK(launch_eval2d(a, k0 + k, cb, max_band, last_ends, ctx->st));
+        CK(launch_eval2d(a, k0 + k, k == 0, cb, max_band, last_ends, ctx->st));
         ctx->launches += 1;
     }
     if (any_2d) {
@@ -1458,7 +1458,7 @@ gcf_status run_fast_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, con
     static_assert(kSteps % 2 == 0, "the final states land in buffer 0");
     const int last_ends = eval_last_ends((long long)nj * max_chunks, ctx->n_sms);
     for (int k = 0; k < kSteps; ++k) {
-        CK(launch_eval2d(a, k, 2, max_band, last_ends, ctx->st));
+        CK(launch_eval2d(a, k, k == 0, 2, max_band, last_ends, ctx->st));
         ctx->launches += 1;
     }
     CK(record_timing(ctx->fev[4], ctx->st));

@@ -538,7 +538,8 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 // One launch is one step of every job's search; consecutive steps are
 // programmatic dependent launches: a step's CTAs start, and load their pixels
 // (which no step writes), while the step before still runs, and wait for it
-// only then.  The state and the sums pass through two buffers by the parity
+// only then.  (The first step of a search waits for all launches before it: one
+// of them writes the pixels' spectrum.)  The state and the sums pass through two buffers by the parity
 // of the step (jin, pin: the launch before's).  Two ways to end a step:
 //
 //  * few CTAs (last_ends = 0): every CTA of the next launch sums the step's
@@ -1433,7 +1434,7 @@ k_table_search(TableArgs A)
 // 1378; 8 (328 CTAs) 2041 and 2055; 12 (492 CTAs) 2845 and 2717.
 int eval_last_ends(long long ctas, int sms) { return ctas > 2LL * sms ? 1 : 0; }
 
-cudaError_t launch_eval2d(const EvalArgs& a, int k, int cand_blocks, int max_band_n, int last_ends,
+cudaError_t launch_eval2d(const EvalArgs& a, int k, bool first, int cand_blocks, int max_band_n, int last_ends,
                           cudaStream_t st)
 {
     if (a.njobs <= 0 || cand_blocks <= 0 || max_band_n < 0) return cudaSuccess;
@@ -1446,7 +1447,7 @@ cudaError_t launch_eval2d(const EvalArgs& a, int k, int cand_blocks, int max_ban
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = first ? 0 : 1;
     const int in = k & 1, out = in ^ 1;
     const size_t np = (size_t)a.njobs * a.max_chunks * kLineCand;
     return cudaLaunchKernelEx(&cfg, k_eval2d, (const SearchJob*)(a.jobs + (size_t)in * a.njobs),
