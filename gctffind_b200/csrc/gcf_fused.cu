@@ -1040,6 +1040,10 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
             for (int ky = tid; ky < FT; ky += S::THR)
                 partial[(size_t)item.w * FCX * FT + (size_t)((ky + FT / 2) & (FT - 1)) * FCX + FT / 2] =
                     accN[ky <= FT / 2 ? ky : FT - ky];
+        // this thread's plain accesses to the column buffer come before the
+        // peers' bulk copies into it, which the next item's cluster barrier
+        // admits (another proxy: the barrier alone does not order them)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
