@@ -42,6 +42,7 @@ EXPORTS = [
     "gcf_get_radial_average", "gcf_rescale_dims", "gcf_rescale", "gcf_run_series",
     "gcf_run_batch", "gcf_mrc_info", "gcf_mrc_read", "gcf_mrc_read_tilts", "gcf_mrc_write",
     "gcf_get_stage_times", "gcf_get_launch_count", "gcf_get_search_counts", "gcf_avg_spectrum_noalloc",
+    "gcf_avg_spectrum_gave_up",
     "gcf_gemm_bf16", "gcf_run_batch_mode", "gcf_get_fast_counts", "gcf_get_fast_times",
     "gcf_nn_param_count", "gcf_nn_init", "gcf_nn_set_params", "gcf_nn_get_params", "gcf_nn_save",
     "gcf_nn_load", "gcf_set_learned_threshold", "gcf_set_rescale_impl", "gcf_nn_train", "gcf_nn_synth_inputs", "gcf_nn_inputs",
@@ -157,6 +158,7 @@ def load_library(path: str = LIB_PATH):
     L.gcf_get_launch_count.argtypes = [vp, C.POINTER(C.c_longlong)]
     L.gcf_get_search_counts.argtypes = [vp, C.POINTER(C.c_longlong)]
     L.gcf_avg_spectrum_noalloc.argtypes = [vp, i, i, i, vp, vp]
+    L.gcf_avg_spectrum_gave_up.argtypes = [vp, i, i, i, vp, vp]
     ll = C.c_longlong
     L.gcf_gemm_bf16.argtypes = [vp, ll, vp, ll, i, i, i, vp, ll, i, i, vp]
     L.gcf_gemm_bf16_ex.argtypes = [vp, ll, vp, ll, i, i, i, vp, ll, i, i, i, vp]

@@ -678,6 +678,12 @@ k_fused_spectrum(const FusedTab* __restrict__ imgs, const int4* __restrict__ ite
 // warps' time in both).  The barrier that says "the column buffers have been
 // read" is arrived at after a tile's last column loads and waited for after
 // the next tile's first row transforms.
+//
+// A wait that gives up sets *err (the spectra of the launch are void) and tells
+// every CTA of its cluster (s_dead): none of them sends, announces or waits for
+// bytes any more, rank 0 takes no further item, and only the cluster barriers
+// that keep the CTAs together still run.  Every CTA's copies are complete before
+// the last of these, so none lands in shared memory that has been given back.
 template <int CL_, int NW_>
 struct PairShape {
     static constexpr int CL = CL_;                  // CTAs per cluster
@@ -711,8 +717,9 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank)
 }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Waits for the mbarrier phase of the given parity, about a second at most.
-__device__ bool wait_phase(uint32_t bar, uint32_t parity)
+// Waits for the mbarrier phase of the given parity, about a second at most and
+// no longer than until *gave_up is set.
+__device__ bool wait_phase(uint32_t bar, uint32_t parity, const volatile int* gave_up)
 {
     unsigned long long t0 = 0;
     for (uint32_t it = 0;; ++it) {
@@ -726,6 +733,7 @@ __device__ bool wait_phase(uint32_t bar, uint32_t parity)
             : "memory");
         if (ok) return true;
         if ((it & 63) == 63) {
+            if (*gave_up) return false;
             unsigned long long now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
             if (t0 == 0) t0 = now;
@@ -766,7 +774,8 @@ template <class S>
 __global__ void __launch_bounds__(S::THR, S::MINB)
 k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict__ items, int nitems,
                       const float* __restrict__ taper, const float2* __restrict__ twg,
-                      float* __restrict__ partial, unsigned long long* __restrict__ next_item, int* __restrict__ err)
+                      float* __restrict__ partial, unsigned long long* __restrict__ next_item, int* __restrict__ err,
+                      uint32_t tile_bytes)   // bytes a tile brings to a CTA's column buffer: S::BUF
 {
     extern __shared__ __align__(16) unsigned char smem[];
     float2* colbuf = reinterpret_cast<float2*>(smem);
@@ -777,7 +786,9 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
 
     __shared__ int s_item[2];   // the item rank 0 fetched, by item parity
     __shared__ uint32_t s_tmem;
+    __shared__ int s_dead;      // a wait of this cluster gave up
     __shared__ __align__(8) unsigned long long s_bar;   // the column buffer's bytes of one tile
+    const volatile int* const dead = &s_dead;
     cg::cluster_group cluster = cg::this_cluster();
     const int r = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -794,6 +805,7 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
+        s_dead = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -821,11 +833,10 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
 
     int ipar = 0;       // s_item parity
     uint32_t phase = 0; // of s_bar: one per tile
-    bool dead = false;  // a wait gave up: no further waits (the results are void, err is set)
     for (;;) {
         // as in k_fused_spectrum: items in order from one counter, each slot
         // rewritten two items later
-        if (r == 0 && tid == 0) s_item[ipar] = take_front(next_item, nitems);
+        if (r == 0 && tid == 0) s_item[ipar] = *dead ? nitems : take_front(next_item, nitems);
         cluster.sync();
         const int it = *cluster.map_shared_rank(&s_item[ipar], 0);
         ipar ^= 1;
@@ -886,9 +897,8 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
         load_rows(src + half_rows);
 
         for (int t = item.y; t < item.z; ++t) {
-            if (tid == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                             "r"((uint32_t)S::BUF)
+            if (tid == 0 && !*dead)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tile_bytes)
                              : "memory");
             const int t1 = t + 1 < item.z ? t + 1 : t;
             const float* src1 = rows_of(t1);
@@ -949,7 +959,7 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (q == 0 && t > item.y) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-                if (lane < S::CL) {
+                if (lane < S::CL && !*dead) {
                     const uint32_t block = smem_addr(colbuf + (size_t)(S::R / 4 * r + warp + q * S::NW) * S::BLOCK);
                     asm volatile(
                         "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -962,9 +972,9 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
             }
             sent();
             // every block of this tile has landed in the column buffer
-            if (!dead && !wait_phase(bar, phase)) {
-                dead = true;
-                if (err) atomicExch(err, 8);
+            if (!*dead && !wait_phase(bar, phase, dead)) {
+                atomicExch(err, 8);
+                for (int k = 0; k < S::CL; ++k) *cluster.map_shared_rank(&s_dead, k) = 1;
             }
             phase ^= 1;
 
@@ -1046,6 +1056,7 @@ k_fused_spectrum_pair(const FusedTab* __restrict__ imgs, const int4* __restrict_
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // this thread's copies have arrived
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster.sync();   // keep shared memory alive until every peer is done
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1338,14 +1349,16 @@ cudaError_t max_pair_clusters(int* n)
 
 template <class S>
 cudaError_t launch_pair(int nclusters, cudaStream_t st, const void* descs, const int4* items, int nitems,
-                        const float* taper, const float2* tw, float* partial, unsigned long long* next_item, int* err)
+                        const float* taper, const float2* tw, float* partial, unsigned long long* next_item, int* err,
+                        uint32_t extra_bytes)
 {
+    if (!err) return cudaErrorInvalidValue;
     cudaError_t e = prepare_pair<S>();
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = pair_cfg<S>(nclusters, st, attr);
     return cudaLaunchKernelEx(&cfg, k_fused_spectrum_pair<S>, reinterpret_cast<const FusedTab*>(descs), items, nitems,
-                              taper, tw, partial, next_item, err);
+                              taper, tw, partial, next_item, err, (uint32_t)S::BUF + extra_bytes);
 }
 
 template <class S>
@@ -1591,7 +1604,7 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
                          int nitems, const int* first, const int* group, const float* inv, int img0, int nimg,
                          const float* taper, const float2* tw, float* partial, float* raw,
                          unsigned long long* next_item, int* err, int nclusters, int shape, cudaStream_t st,
-                         cudaEvent_t ev0, cudaEvent_t ev1, const SoloLaunch* solo)
+                         cudaEvent_t ev0, cudaEvent_t ev1, const SoloLaunch* solo, unsigned extra_bytes)
 {
     if (nclusters < 1) nclusters = 1;
     // few blocks: one per SM, bound by how many loads it has in flight, so 1024
@@ -1632,7 +1645,7 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
         e = cudaLaunchKernelEx(&cfg, k_fused_spectrum<Shape8W16>, reinterpret_cast<const FusedTab*>(descs),
                                items, nitems, taper, tw, partial, next_item);
     } else {
-        e = launch_pair<Pair8>(nclusters, st, descs, items, nitems, taper, tw, partial, next_item, err);
+        e = launch_pair<Pair8>(nclusters, st, descs, items, nitems, taper, tw, partial, next_item, err, extra_bytes);
     }
     if (e != cudaSuccess) return e;
     if (use_solo) {
@@ -1762,10 +1775,13 @@ gcf_status na_setup(int dev, unsigned char** base, int* clusters)
 }  // namespace
 }  // namespace gcf
 
-extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, int height, int pitch,
-                                               float* dev_raw_out, void* cuda_stream)
+namespace gcf {
+namespace {
+
+// extra_bytes: see launch_fused
+gcf_status na_spectrum(const float* dev_img, int width, int height, int pitch, float* dev_raw_out, cudaStream_t st,
+                       unsigned extra_bytes)
 {
-    using namespace gcf;
     if (!dev_img || !dev_raw_out || width < FT || height < FT || pitch < width)
         return GCF_ERR_INVALID_ARG;
     // tile layout of CGenAvgSpectrum::SetSizes (FindCTF/CGenAvgSpectrum.cpp:40-75)
@@ -1780,7 +1796,6 @@ extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, 
     int clusters = 0;
     gcf_status s = na_setup(dev, &base, &clusters);
     if (s != GCF_OK) return s;
-    cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     NaMeta meta;
     std::memset(&meta, 0, sizeof(meta));
     double* bsum = reinterpret_cast<double*>(base + kNaBsumOff);
@@ -1818,7 +1833,22 @@ extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, 
                                  reinterpret_cast<const float*>(base + kNaTaperOff),
                                  reinterpret_cast<const float2*>(base + kNaTwOff),
                                  reinterpret_cast<float*>(base), dev_raw_out, &dmeta->next_item, &dmeta->err, ncl,
-                                 g_na_shape[dev], st, nullptr, nullptr);
+                                 g_na_shape[dev], st, nullptr, nullptr, nullptr, extra_bytes);
     if (e != cudaSuccess) return GCF_ERR_CUDA;
     return GCF_OK;
+}
+
+}  // namespace
+}  // namespace gcf
+
+extern "C" gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, int height, int pitch,
+                                               float* dev_raw_out, void* cuda_stream)
+{
+    return gcf::na_spectrum(dev_img, width, height, pitch, dev_raw_out, static_cast<cudaStream_t>(cuda_stream), 0);
+}
+
+extern "C" gcf_status gcf_avg_spectrum_gave_up(const float* dev_img, int width, int height, int pitch,
+                                               float* dev_raw_out, void* cuda_stream)
+{
+    return gcf::na_spectrum(dev_img, width, height, pitch, dev_raw_out, static_cast<cudaStream_t>(cuda_stream), 16);
 }

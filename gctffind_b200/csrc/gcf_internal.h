@@ -249,11 +249,14 @@ size_t solo_scratch_floats(int nsolo);
 // item (see k_item_reduce), 1 for whole items; inv[img] = 1 / tiles of img; raw: the spectrum of image img0;
 // next_item: the launch's 64-bit item queue counter (zeroed on st).
 // err: device flag, set when a bounded wait gave up (the spectra are void).
+// extra_bytes: bytes that the pair kernel's CTAs wait for beyond those that
+// are sent; not 0 only to make these waits run out.
 cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blocks, const int4* items,
                          int nitems, const int* first, const int* group, const float* inv, int img0, int nimg,
                          const float* taper, const float2* tw, float* partial, float* raw,
                          unsigned long long* next_item, int* err, int nclusters, int shape, cudaStream_t st,
-                         cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, const SoloLaunch* solo = nullptr);
+                         cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, const SoloLaunch* solo = nullptr,
+                         unsigned extra_bytes = 0);
 
 // gcf_post.cu
 // ctf = raw minus its box mean, and mom[m] = (mean, second moment) of ctf.

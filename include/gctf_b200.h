@@ -464,6 +464,11 @@ gcf_status gcf_gemm_bf16_ex(const void* a, long long lda, const void* b, long lo
  * other threads) race and must be serialised by the caller. */
 gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, int height, int pitch,
                                     float* dev_raw_out, void* cuda_stream);
+/* The same call with its clusters waiting for bytes that nobody sends, so that
+ * every bounded wait runs out (after about a second): what a caller sees of a
+ * wait that gave up, for tests. */
+gcf_status gcf_avg_spectrum_gave_up(const float* dev_img, int width, int height, int pitch,
+                                    float* dev_raw_out, void* cuda_stream);
 
 /* Device time (ms, CUDA events on the context streams) of the stages of the
  * last batched call: [0] upload of host inputs (it overlaps [2]), [1] time
