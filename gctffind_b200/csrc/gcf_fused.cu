@@ -1233,9 +1233,12 @@ k_fused_spectrum_solo(const FusedTab* __restrict__ imgs, const int4* __restrict_
 // raw[img] = sum of the img's item partials (in item order) / ntiles / 2.
 // group[img] > 1: each partial is one tile, and that many consecutive ones make
 // an item; their FP32 sum, in tile order, is what a cluster that takes the
-// whole item accumulates, bit for bit.
+// whole item accumulates, bit for bit.  Where a bounded wait gave up (*err), the
+// partials are void and so is the spectrum: NaN throughout, for callers that
+// have no other sign of it (gcf_avg_spectrum_noalloc).
 __global__ void k_item_reduce(const float* __restrict__ partial, const int* __restrict__ first,
-                              const int* __restrict__ group, const float* __restrict__ inv, float* __restrict__ raw)
+                              const int* __restrict__ group, const float* __restrict__ inv,
+                              const int* __restrict__ err, float* __restrict__ raw)
 {
     const int n = FCX * FT;
     int img = blockIdx.y;
@@ -1255,6 +1258,7 @@ __global__ void k_item_reduce(const float* __restrict__ partial, const int* __re
             s += f;
         }
     }
+    if (*err) s = __longlong_as_double(0x7ff8000000000000ll);
     raw[(size_t)img * n + i] = (float)(s * (double)inv[img] * 0.5);   // rows were split without the 1/2
 }
 
@@ -1663,7 +1667,7 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
     }
     if (ev1 && (e = record_timing(ev1, st)) != cudaSuccess) return e;
     dim3 g((FCX * FT + 255) / 256, nimg);
-    k_item_reduce<<<g, 256, 0, st>>>(partial, first + img0, group ? group + img0 : nullptr, inv + img0, raw);
+    k_item_reduce<<<g, 256, 0, st>>>(partial, first + img0, group ? group + img0 : nullptr, inv + img0, err, raw);
     return cudaGetLastError();
 }
 

@@ -248,7 +248,8 @@ size_t solo_scratch_floats(int nsolo);
 // image img; group (nullable): items of img that are single tiles of one
 // item (see k_item_reduce), 1 for whole items; inv[img] = 1 / tiles of img; raw: the spectrum of image img0;
 // next_item: the launch's 64-bit item queue counter (zeroed on st).
-// err: device flag, set when a bounded wait gave up (the spectra are void).
+// err: device flag, set when a bounded wait gave up: the spectra are void and
+// come out as NaN.
 // extra_bytes: bytes that the pair kernel's CTAs wait for beyond those that
 // are sent; not 0 only to make these waits run out.
 cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blocks, const int4* items,

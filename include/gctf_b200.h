@@ -461,7 +461,10 @@ gcf_status gcf_gemm_bf16_ex(const void* a, long long lda, const void* b, long lo
  * The first call on a device finds the array's address and fills its
  * constant tables; make that first call before any stream capture.  All
  * calls share the array: calls that overlap on the GPU (other streams,
- * other threads) race and must be serialised by the caller. */
+ * other threads) race and must be serialised by the caller.
+ * The call returns before its kernels have run.  If a bounded wait in one of
+ * them gives up (a cluster that makes no progress for about a second), the
+ * whole spectrum is NaN. */
 gcf_status gcf_avg_spectrum_noalloc(const float* dev_img, int width, int height, int pitch,
                                     float* dev_raw_out, void* cuda_stream);
 /* The same call with its clusters waiting for bytes that nobody sends, so that

@@ -32,3 +32,15 @@ def test_kernel_ends_soon_after_a_wait_gives_up(gpu_lib, w, h):
         _call(L, "gcf_avg_spectrum_gave_up", img, out)
         assert 0.5 < time.monotonic() - t < 5.0
         assert torch.equal(_call(L, "gcf_avg_spectrum_noalloc", img, out), want)
+
+
+def test_spectrum_of_a_wait_that_gave_up_is_nan(gpu_lib):
+    """The allocation-free call cannot report it in its status, which it returns
+    before the kernels run."""
+    import torch
+    L = gpu_lib.load_library()
+    img = torch.ones((1200, 1100), device="cuda")
+    img[::3, ::5] = 4.0
+    out = torch.zeros((512, 257), device="cuda")
+    assert torch.isnan(_call(L, "gcf_avg_spectrum_gave_up", img, out)).all()
+    assert torch.isfinite(_call(L, "gcf_avg_spectrum_noalloc", img, out)).all()
