@@ -338,52 +338,84 @@ struct FusedTab {
 // of GCalcMoment2D (Util/GCalcMoment2D.cu:10-58) without a second read.
 // Each warp sums whole block rows with 16-byte loads when the rows are
 // 16-byte aligned (4 independent FP64 partial sums per lane keep several
-// loads in flight); otherwise it falls back to 4-byte loads.
-__global__ void __launch_bounds__(1024) k_block_sums(const FusedTab* __restrict__ imgs,
-                                                     double* const* __restrict__ out)
+// loads in flight); otherwise it falls back to 4-byte loads.  The rows of a
+// block are summed in kSumRows interleaved groups whatever the number of
+// warps, so that a sum does not depend on the launch's other images.
+constexpr int kSumRows = 32;
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) k_block_sums(const FusedTab* __restrict__ imgs,
+                                                        double* const* __restrict__ out)
 {
-    __shared__ double sh[32];
+    constexpr int GW = kSumRows / NW;   // row groups per warp: warp, warp + NW, ...
+    constexpr int S = FT / 2;           // block rows and columns: the tiles' stride
+    static_assert((GW == 1 || GW == 4) && S % kSumRows == 0, "whole groups, and the reduction below");
+    __shared__ double sh[kSumRows];
     const FusedTab im = imgs[blockIdx.y];
     const int nby = im.nty + 1;
     const int b = blockIdx.x;
     if (b >= im.nbx * nby) return;
-    const int bx = b % im.nbx, by = b / im.nbx, S = im.stride;
+    const int bx = b % im.nbx, by = b / im.nbx;
     const float* src = im.img + (size_t)(im.offy + by * S) * im.pitch + im.offx + bx * S;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const bool v4 = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (im.pitch % 4 == 0) && (S % 4 == 0);
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool v4 = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && (im.pitch % 4 == 0);
+    double s[GW][4];
+#pragma unroll
+    for (int g = 0; g < GW; ++g) s[g][0] = s[g][1] = s[g][2] = s[g][3] = 0.0;
+    // all groups of the warp at once, so that several loads per thread are in
+    // flight: 41 micrographs of 4096 x 4096 (2.75 GB, bound by HBM) in 0.38 ms,
+    // 0.56 ms with one group after the other
     if (v4) {
-        const int q = S / 4;   // float4 per block row
-        // unrolled so that several 16-byte loads per thread are in flight
-        // (the additions keep their order): 2.75 GB in 0.42 ms, the measured
-        // copy bandwidth, against 0.53 ms with one load in flight
-#pragma unroll 4
-        for (int y = warp; y < S; y += nw) {
-            const float4* row = reinterpret_cast<const float4*>(src + (size_t)y * im.pitch);
-#pragma unroll 2
-            for (int x = lane; x < q; x += 32) {
-                float4 v = __ldg(row + x);
-                s0 += (double)v.x;
-                s1 += (double)v.y;
-                s2 += (double)v.z;
-                s3 += (double)v.w;
+        const size_t step = (size_t)NW * im.pitch / 4;
+        for (int y = warp; y < S; y += kSumRows) {
+            const float4* row = reinterpret_cast<const float4*>(src + (size_t)y * im.pitch) + lane;
+#pragma unroll
+            for (int x = 0; x < S / 4; x += 32) {
+#pragma unroll
+                for (int g = 0; g < GW; ++g) {
+                    const float4 v = __ldg(row + g * step + x);
+                    s[g][0] += (double)v.x;
+                    s[g][1] += (double)v.y;
+                    s[g][2] += (double)v.z;
+                    s[g][3] += (double)v.w;
+                }
             }
         }
     } else {
-        for (int y = warp; y < S; y += nw) {
-            const float* row = src + (size_t)y * im.pitch;
-            for (int x = lane; x < S; x += 32) s0 += (double)__ldg(row + x);
+        const size_t step = (size_t)NW * im.pitch;
+        for (int y = warp; y < S; y += kSumRows) {
+            const float* row = src + (size_t)y * im.pitch + lane;
+#pragma unroll 4
+            for (int x = 0; x < S; x += 128) {
+#pragma unroll
+                for (int g = 0; g < GW; ++g)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[g][k] += (double)__ldg(row + g * step + x + 32 * k);
+            }
         }
     }
-    double s = (s0 + s1) + (s2 + s3);
+    double t[GW];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) sh[warp] = s;
+    for (int g = 0; g < GW; ++g) t[g] = (s[g][0] + s[g][1]) + (s[g][2] + s[g][3]);
+    // each group's sum over the lanes, by halves: of four groups a lane keeps
+    // two, then one (6 exchanges, not 20)
+    const bool up = GW > 1 && (lane & 16), vp = GW > 1 && (lane & 8);
+    double r = t[0];
+    if constexpr (GW == 4) {
+        const double a0 = (up ? t[2] : t[0]) + __shfl_xor_sync(0xffffffffu, up ? t[0] : t[2], 16);
+        const double a1 = (up ? t[3] : t[1]) + __shfl_xor_sync(0xffffffffu, up ? t[1] : t[3], 16);
+        r = (vp ? a1 : a0) + __shfl_xor_sync(0xffffffffu, vp ? a0 : a1, 8);
+    } else {
+        r += __shfl_xor_sync(0xffffffffu, r, 16);
+        r += __shfl_xor_sync(0xffffffffu, r, 8);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if ((lane & 7) == 0) sh[warp + NW * (2 * up + vp)] = r;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < nw; ++w) t += sh[w];
-        out[blockIdx.y][b] = t;
+        double v = 0.0;
+        for (int g = 0; g < kSumRows; ++g) v += sh[g];
+        out[blockIdx.y][b] = v;
     }
 }
 
@@ -1612,12 +1644,13 @@ cudaError_t launch_fused(const void* descs, double* const* bsum_out, int max_blo
 {
     if (nclusters < 1) nclusters = 1;
     // few blocks: one per SM, bound by how many loads it has in flight, so 1024
-    // threads (1024 x 1024 frame, 16 blocks: 14.1 -> 6.5 us; 2048 x 2048, 64:
-    // 20.8 -> 8.4 us); many:
-    // 256, eight blocks per SM
-    const int block = (long long)max_blocks * nimg <= 148 ? 1024 : 256;
-    k_block_sums<<<dim3(max_blocks, nimg), block, 0, st>>>(reinterpret_cast<const FusedTab*>(descs) + img0,
-                                                          bsum_out + img0);
+    // threads (1024 x 1024 frame, 16 blocks: 14.1 us with 256 threads, 5.6 with
+    // 1024; 2048 x 2048, 64: 20.8 and 6.8 us); many: 256, four blocks per SM
+    const auto* tabs = reinterpret_cast<const FusedTab*>(descs) + img0;
+    if ((long long)max_blocks * nimg <= 148)
+        k_block_sums<32><<<dim3(max_blocks, nimg), 1024, 0, st>>>(tabs, bsum_out + img0);
+    else
+        k_block_sums<8><<<dim3(max_blocks, nimg), 256, 0, st>>>(tabs, bsum_out + img0);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(next_item, 0, sizeof(unsigned long long), st)) != cudaSuccess) return e;
