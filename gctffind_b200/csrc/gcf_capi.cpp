@@ -1177,11 +1177,15 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     CK(ctx->best_1d.ensure((size_t)nj * ctas_1d));
     CK(ctx->first_1d.ensure(nj));
     // Upper bound of non-empty steps: CC0 + astigmatism grid + 19 x 4
-    // refinements; one more launch ends the last of them.  The state buffers
-    // alternate, so that the last launch writes buffer 0.
+    // refinements; where a step's CTAs do not end it themselves, one more
+    // launch ends the last of them.  The state buffers alternate, so that the
+    // last launch writes buffer 0.
     bool any_2d = false;
     for (const JobSpec& s : specs) any_2d = any_2d || s.mode <= 1;
-    const int steps = any_2d ? 3 + 19 * ((any_grid ? 2 : 0) + 1 + (any_phase ? 1 : 0)) : 0;
+    const long long per_y = (long long)nj * max_chunks;
+    const int last_ends = eval_last_ends(per_y, ctx->n_sms);
+    const int steps =
+        any_2d ? 2 + 19 * ((any_grid ? 2 : 0) + 1 + (any_phase ? 1 : 0)) + (last_ends ? 0 : 1) : 0;
     const int k0 = steps & 1;
     SearchJob* const jobs0 = ctx->jobs.p + (size_t)k0 * nj;
     CK(cudaMemsetAsync(ctx->arrive.p, 0, (size_t)nj * (1 + kMaxCandBlocks) * sizeof(int), ctx->st));
@@ -1207,8 +1211,6 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
     // candidates and exit.  Enough for about four CTAs per SM where the last
     // CTA ends a step (8 jobs 2040 us against 2164 us with enough for six),
     // two where every CTA does (4 jobs 1203 us against 1368 us with four).
-    const long long per_y = (long long)nj * max_chunks;
-    const int last_ends = eval_last_ends(per_y, ctx->n_sms);
     const long long want = (last_ends ? 4LL : 2LL) * ctx->n_sms;
     const int line_cb = (int)std::min<long long>(4, std::max<long long>(1, (want + per_y - 1) / per_y));
     for (int k = 0; k < steps; ++k) {

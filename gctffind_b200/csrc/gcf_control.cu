@@ -542,7 +542,7 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 // of them writes the pixels' spectrum.)  The state and the sums pass through two buffers by the parity
 // of the step (jin, pin: the launch before's).  Two ways to end a step:
 //
-//  * few CTAs (last_ends = 0): every CTA of the next launch sums the step's
+//  * few CTAs (kFew): every CTA of the next launch sums the step's
 //    partial sums (up to kLineCand x chunks), advances its own copy of the
 //    job's state machine and makes its own candidates.  A step of one job is
 //    a chain of latencies, not work: with the job's last CTA ending each
@@ -552,23 +552,30 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 //    step it stays in their instruction caches, the state and the sums are
 //    read at once, and four warps share a candidate's slow parts (double sine,
 //    cosine and divisions): 8.5 us per step.
-//  * many CTAs (last_ends = 1): the same work in every CTA would cost more
+//  * many CTAs (kMany; kManyFirst for the search's first step, which makes its
+//    own candidates): the same work in every CTA would cost more
 //    than it saves (96 searches at once: 18.6 ms against 16.1 ms), so the
 //    job's last CTA to finish (an arrival counter, no waiting) ends the step
-//    and writes the next candidates.
+//    and writes the next candidates.  A kernel of its own: with both ways, or
+//    only the first step's, in one kernel the line steps of 256 searches took
+//    242 us each, not 234 (96: 97 us, not 94).
 //
 // In both, the astigmatism grid's 2601 candidates are summed by the last CTA
 // of each candidate block y, in parallel over y, not by one CTA.
 constexpr int kFastCand = 64;   // candidates whose sums are read before their count is known
 
+enum class Steps { kFew, kManyFirst, kMany };
+
+template <Steps kSteps>
 __global__ void __launch_bounds__(kEvalThreads, 3)
 k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const BandDev* __restrict__ bands,
          const float* __restrict__ band_spec, const int2* __restrict__ spec_off, const double* __restrict__ sum_ss,
          const double2* __restrict__ pin, double2* __restrict__ pout, double2* __restrict__ pgrid, int max_chunks,
          float4* __restrict__ cand, int* __restrict__ arrive, int* __restrict__ arrive_y,
          BestCand* __restrict__ best_y, const BestCand* __restrict__ best_in,
-         BestCand* __restrict__ best_out, int last_ends)
+         BestCand* __restrict__ best_out)
 {
+    constexpr bool kLastEnds = kSteps != Steps::kFew;
     __shared__ float4 sq[kEvalCB];
     __shared__ float red[kEvalThreads / 32][2 * kEvalCB];
     __shared__ double2 shs[kEvalThreads];
@@ -617,7 +624,7 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
     const int* const jw = reinterpret_cast<const int*>(jin + j);
     int kind, ncand;
     bool fresh;
-    if (!last_ends) {
+    if constexpr (!kLastEnds) {
         // the state and the first kFastCand candidates' sums come in together
         // (whether that many are there or not), four threads per candidate
         const int u = threadIdx.x & (kFastCand - 1), q = threadIdx.x / kFastCand;
@@ -683,20 +690,17 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
     } else {
         kind = __ldcg(&jin[j].step);
         ncand = __ldcg(&jin[j].ncand);
-        fresh = __ldcg(&jin[j].fresh) != 0;
+        fresh = kSteps == Steps::kManyFirst;
         if (fresh || kind == STEP_DONE) {
             if (threadIdx.x < kJobWords) reinterpret_cast<int*>(&sJ)[threadIdx.x] = __ldcg(jw + threadIdx.x);
             __syncthreads();
-            if (kind == STEP_DONE) {   // passed on; a fresh state is written by the step's last CTA
-                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
-                    reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
-                return;
+            if (fresh && kind != STEP_DONE) {
+                if (threadIdx.x == 0) next_step(sJ, false, 0, ArgMax{0.0f, -1}, 0.0f, s_cval);
+                __syncthreads();
+                kind = sJ.step;
+                ncand = sJ.ncand;
             }
-            if (threadIdx.x == 0) next_step(sJ, false, 0, ArgMax{0.0f, -1}, 0.0f, s_cval);
-            __syncthreads();
-            kind = sJ.step;
-            ncand = sJ.ncand;
-            if (kind == STEP_DONE) {
+            if (kind == STEP_DONE) {   // passed on; a fresh state is written by the step's last CTA
                 if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kJobWords)
                     reinterpret_cast<int*>(jout + j)[threadIdx.x] = reinterpret_cast<const int*>(&sJ)[threadIdx.x];
                 return;
@@ -717,7 +721,7 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
     // candidate blocks y, y + gridDim.y, ... so any candidate count is covered
     for (int c0 = blockIdx.y * kEvalCB; c0 < ncand && nchunk > 0; c0 += gridDim.y * kEvalCB) {
         __syncthreads();
-        if (last_ends && !fresh) {
+        if constexpr (kSteps == Steps::kMany) {
             if (threadIdx.x < kEvalCB) {
                 const int c = c0 + threadIdx.x;
                 sq[threadIdx.x] =
@@ -864,7 +868,7 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
             }
         }
     }
-    if (!last_ends && ncand <= kLineCand) return;   // summed by the next launch's CTAs
+    if (!kLastEnds && ncand <= kLineCand) return;   // summed by the next launch's CTAs
     // arrival: the last CTA of the job, or of its candidate block y (blocks
     // y, y + gridDim.y, ...) where there are many candidates
     const int y = blockIdx.y, gy = gridDim.y, ny = min(gy, cand_blocks), nx = max(nchunk, 1);
@@ -897,7 +901,7 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
         __syncthreads();
         m = block_argmax(m, shm);
     }
-    if (!last_ends) {   // a grid: the next launch's CTAs end it with this
+    if constexpr (!kLastEnds) {   // a grid: the next launch's CTAs end it with this
         if (threadIdx.x == 0) best_out[j] = BestCand{m.v, m.i};
         return;
     }
@@ -1450,11 +1454,14 @@ cudaError_t launch_eval2d(const EvalArgs& a, int k, bool first, int cand_blocks,
     cfg.numAttrs = first ? 0 : 1;
     const int in = k & 1, out = in ^ 1;
     const size_t np = (size_t)a.njobs * a.max_chunks * kLineCand;
-    return cudaLaunchKernelEx(&cfg, k_eval2d, (const SearchJob*)(a.jobs + (size_t)in * a.njobs),
-                              a.jobs + (size_t)out * a.njobs, a.bands, a.band_spec, a.spec_off, a.sum_ss,
-                              (const double2*)(a.part + in * np), a.part + out * np, a.part_grid, a.max_chunks,
-                              a.cand, a.arrive, a.arrive_y, a.best_y, (const BestCand*)(a.best + (size_t)in * a.njobs),
-                              a.best + (size_t)out * a.njobs, last_ends);
+    return cudaLaunchKernelEx(&cfg,
+                              !last_ends ? k_eval2d<Steps::kFew>
+                              : first    ? k_eval2d<Steps::kManyFirst>
+                                         : k_eval2d<Steps::kMany>,
+                              (const SearchJob*)(a.jobs + (size_t)in * a.njobs), a.jobs + (size_t)out * a.njobs,
+                              a.bands, a.band_spec, a.spec_off, a.sum_ss, (const double2*)(a.part + in * np),
+                              a.part + out * np, a.part_grid, a.max_chunks, a.cand, a.arrive, a.arrive_y, a.best_y,
+                              (const BestCand*)(a.best + (size_t)in * a.njobs), a.best + (size_t)out * a.njobs);
 }
 
 int search1d_ctas(int njobs, bool phase, int sms)

@@ -292,14 +292,14 @@ void launch_ctf_res(const float* ctf, int tile, const SearchJob* jobs, int njobs
                     const int* ring_pix, const double2* ring_geo, double* ring_sums, float* cc,
                     cudaStream_t st);
 
-// gcf_control.cu: step k of every job's search: ends step k - 1 and
-// evaluates the next candidates, cand_blocks candidate blocks at a time.
+// gcf_control.cu: step k of every job's search, cand_blocks candidate blocks
+// at a time.  Where last_ends is 0 a launch ends step k - 1 before it evaluates
+// its own candidates, and the launch after the last step ends that one.
 // k picks the buffers by its parity.  Every step but the search's first is
 // programmatically dependent on the step before it: that one may still run
 // when this step's CTAs load what no step writes (bands, band_spec, spec_off).
 // The first step is an ordinary launch, because the launch before it may be
 // the one that writes band_spec (k_band_gather, where no 1D search runs).
-// The launch after the last step ends it.
 cudaError_t launch_eval2d(const EvalArgs& a, int k, bool first, int cand_blocks, int max_band_n, int last_ends,
                           cudaStream_t st);
 // Whether the last CTA of a step ends it and makes the next candidates (else
