@@ -449,44 +449,55 @@ __device__ ArgMax block_argmax(ArgMax m, ArgMax* sh)
 }
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
+constexpr int kFastCand = 64;   // candidates whose sums are read before their count is known
+constexpr int kStrands = 4;     // strands of a candidate's sum over the chunks
+static_assert(kEvalThreads == kFastCand * kStrands, "a thread per strand");
+
+__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+
 // Best of the candidates of job j's pending step that lie in the candidate
 // blocks y, y + gy, ... (n of them, counted up to whole blocks; those at or
 // beyond ncand do not exist): sums the chunks' partial sums of each (part:
 // [chunk][pitch], so the threads of a warp read adjacent candidates) and
 // keeps the first strict maximum in index order.  One round takes np (a
-// power of two >= n, at most the block size) candidates; the blockDim / np
-// threads of a candidate share its chunks, each with several loads in flight.
+// power of two >= n, 64 at least and the block size at most) candidates; the
+// blockDim / np threads of a candidate share its chunks, each with several
+// loads in flight.  A candidate's chunks are always added as four strands
+// (every fourth chunk) s_t, (s_0 + s_2) + (s_1 + s_3), by however many threads:
+// the sum does not depend on how a step is ended, nor on the step's other jobs.
 __device__ ArgMax reduce_candidates(int n, int y, int gy, int ncand, const double2* __restrict__ part, int pitch,
                                     int nch, double ss, double2* shs, ArgMax* shm, float* cc0)
 {
-    int np = 1;
+    int np = kFastCand;
     while (np < n && np < kEvalThreads) np <<= 1;
     const int G = kEvalThreads / np, u = threadIdx.x & (np - 1), q = threadIdx.x / np;
     ArgMax m{(float)-1e20, -1};
     for (int u0 = 0; u0 < n; u0 += np) {
-        double cs = 0.0, cc = 0.0;
         const int c = (y + (u0 + u) / kEvalCB * gy) * kEvalCB + (u0 + u) % kEvalCB;
         const bool have = u0 + u < n && c < ncand;
-        if (have) {
-            const double2* p = part + c;
+        auto strand = [&](int t) {
+            double2 r = make_double2(0.0, 0.0);
 #pragma unroll 8
-            for (int k = q; k < nch; k += G) {
-                const double2 v = __ldcg(p + (size_t)k * pitch);
-                cs += v.x;
-                cc += v.y;
+            for (int k = t; k < nch; k += kStrands) {
+                const double2 v = __ldcg(part + c + (size_t)k * pitch);
+                r.x += v.x;
+                r.y += v.y;
             }
+            return r;
+        };
+        double2 r = make_double2(0.0, 0.0);
+        if (have) {
+            r = strand(q);
+            if (G < kStrands) r = r + strand(q + 2);
+            if (G == 1) r = r + (strand(1) + strand(3));
         }
         if (G > 1) {   // one round only: np >= n
-            shs[threadIdx.x] = make_double2(cs, cc);
+            shs[threadIdx.x] = r;
             __syncthreads();
             if (q == 0)
-                for (int k = 1; k < G; ++k) {
-                    const double2 v = shs[u + k * np];
-                    cs += v.x;
-                    cc += v.y;
-                }
+                r = G == kStrands ? (r + shs[u + 2 * np]) + (shs[u + np] + shs[u + 3 * np]) : r + shs[u + np];
         }
+        const double cs = r.x, cc = r.y;
         if (q == 0 && have) {
             const double d = sqrt(cc * ss);
             const float ccv = (d == 0.0) ? 0.0f : (float)(cs / d);   // GCC2D mGCalc1D, FindCTF/GCC2D.cu:81-87
@@ -562,8 +573,6 @@ __device__ __noinline__ void next_step(SearchJob& J, bool ended, int n, ArgMax m
 //
 // In both, the astigmatism grid's 2601 candidates are summed by the last CTA
 // of each candidate block y, in parallel over y, not by one CTA.
-constexpr int kFastCand = 64;   // candidates whose sums are read before their count is known
-
 enum class Steps { kFew, kManyFirst, kMany };
 
 template <Steps kSteps>
@@ -628,12 +637,11 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
         // the state and the first kFastCand candidates' sums come in together
         // (whether that many are there or not), four threads per candidate
         const int u = threadIdx.x & (kFastCand - 1), q = threadIdx.x / kFastCand;
-        constexpr int G = kEvalThreads / kFastCand;
         const double2* p = pin + (size_t)j * max_chunks * kLineCand + u;
         const int word = threadIdx.x < kJobWords ? __ldcg(jw + threadIdx.x) : 0;
         double cs = 0.0, cc = 0.0;
 #pragma unroll 10
-        for (int k = q; k < nchunk; k += G) {
+        for (int k = q; k < nchunk; k += kStrands) {
             const double2 v = __ldcg(p + (size_t)k * kLineCand);
             cs += v.x;
             cc += v.y;
@@ -658,13 +666,10 @@ k_eval2d(const SearchJob* __restrict__ jin, SearchJob* __restrict__ jout, const 
                 static_assert(kFastCand == 64, "two warps choose");
                 if (threadIdx.x < kFastCand) {
                     if (u < ncand) {
-#pragma unroll
-                        for (int g = 1; g < G; ++g) {
-                            cs += shs[u + g * kFastCand].x;
-                            cc += shs[u + g * kFastCand].y;
-                        }
-                        const double d = sqrt(cc * sum_ss[j]);
-                        const float v = (d == 0.0) ? 0.0f : (float)(cs / d);   // GCC2D mGCalc1D
+                        const double2 r = (shs[u] + shs[u + 2 * kFastCand]) +
+                                          (shs[u + kFastCand] + shs[u + 3 * kFastCand]);
+                        const double d = sqrt(r.y * sum_ss[j]);
+                        const float v = (d == 0.0) ? 0.0f : (float)(r.x / d);   // GCC2D mGCalc1D
                         if (u == 0) s_cc0 = v;
                         if (v > m.v) m = ArgMax{v, u};
                     }
