@@ -59,7 +59,11 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh /* 32*NV *
 // the Hermitian edge, GRmBackground2D.cu:42-64) go to shared memory, threads
 // slide the vertical box down the columns, then the horizontal one along the
 // rows (one lane per row, odd pitches: no bank conflicts), and the block
-// writes its rows.  All intermediate sums stay in shared memory; the last
+// writes its rows.  The block's shape depends on the number of spectra, its
+// sums do not: float32 values (24 bits) summed over up to 137 x 137 (2^14.2) of
+// them are exact in FP64 (53 bits) in any order while the largest value in reach
+// is below 2^14 times the smallest but zero (2^18 for the 35 x 35 of tile 512;
+// twice the exponent in the spectrum itself, whose square roots these are).  All intermediate sums stay in shared memory; the last
 // block of a spectrum adds the blocks' moments in block order.
 //
 // Bound: latency for few spectra; for many conversions to FP64 and shared-memory
