@@ -462,7 +462,8 @@ __global__ void k_concat(const __nv_bfloat16* __restrict__ x1, const __nv_bfloat
 // outputs and dz once per 32 inputs, and added its slices with atomics: 931 us
 // per step of 256 samples; these two kernels take 132 us.  Relative error
 // against FP64 sums: 1.1e-7 for a million rows x 16 columns (4.6e-7 before),
-// 7.5e-8 for 262144 x 144 (2.6e-7), 3.6e-8 for 6400 x 288 (1.1e-7).
+// 7.5e-8 for 262144 x 144 (2.6e-7), 3.6e-8 for 6400 x 288 (1.1e-7); 2.3e-8 for 64
+// rows (2.4e-8), below which k_wgrad_few takes the layer.
 //
 // A CTA takes 32 outputs x KT columns and a slice of rows, in chunks through
 // a ring of kWgStages shared-memory stages (cp.async, 16 bytes).  Its eight
@@ -630,6 +631,45 @@ __global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ par
     dw[i] = (float)s;
 }
 
+// The same for fewer rows than a chunk of k_wgrad (the dense layers of a batch
+// below 64): one slice would leave the FP64 stage nothing to add, and the tensor
+// core's truncated sums would be all there is (1.25 times the error of a scalar
+// FP32 sum at 17 rows).  The products of BF16 values are exact, their FP64 sums
+// rounded once.  A thread takes one column and kFewOut outputs.  Bound: latency
+// along the rows (all layers' gradients of 33 samples 68 us, 73 with k_wgrad
+// throughout; of 63 samples 87 and 82 us).
+constexpr int kFewRows = 64, kFewOut = 8;
+
+__global__ void __launch_bounds__(256)
+k_wgrad_few(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16* __restrict__ x, long long ldx,
+            int rows, int nout, int nin, float* __restrict__ dw)
+{
+    __shared__ double sz[kFewRows][kFewOut];
+    const int o0 = blockIdx.y * kFewOut, k = blockIdx.x * 256 + threadIdx.x;
+    for (int i = threadIdx.x; i < rows * kFewOut; i += 256) {
+        const int r = i / kFewOut, o = o0 + i % kFewOut;
+        sz[r][i % kFewOut] = o < nout ? (double)bf(dz[(size_t)r * ldz + o]) : 0.0;
+    }
+    __syncthreads();
+    if (k < nin) {
+        double acc[kFewOut] = {};
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r) {
+            const double v = (double)bf(x[(size_t)r * ldx + k]);
+#pragma unroll
+            for (int j = 0; j < kFewOut; ++j) acc[j] = fma(sz[r][j], v, acc[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < kFewOut; ++j)
+            if (o0 + j < nout) dw[(size_t)(o0 + j) * nin + k] = (float)acc[j];
+    }
+    if (blockIdx.x == 0 && threadIdx.x < kFewOut && o0 + (int)threadIdx.x < nout) {
+        double b = 0.0;
+        for (int r = 0; r < rows; ++r) b += sz[r][threadIdx.x];
+        dw[(size_t)nout * nin + o0 + threadIdx.x] = (float)b;
+    }
+}
+
 // Mean squared error over the 3 outputs: loss (atomic) and
 // dpred = 2 (pred - target) / (3 B) as BF16 rows of pitch 8 (zero padded).
 __global__ void k_mse(const float* __restrict__ pred, long long ldp, const float* __restrict__ target, int B,
@@ -780,11 +820,17 @@ static cudaError_t wgrad_shape(const __nv_bfloat16* dz, long long ldz, const __n
     return cudaGetLastError();
 }
 
-// Column tile by the layer's width: 16 (the first layer), 144 up to that
-// width or where 288 would leave most of a tile empty (256), else 288.
+// Few rows: see k_wgrad_few.  Else the column tile by the layer's width: 16
+// (the first layer), 144 up to that width or where 288 would leave most of a
+// tile empty (256), else 288.
 cudaError_t launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows,
                          int nout, int nin, float* scratch, float* dw, cudaStream_t st)
 {
+    if (rows < kFewRows) {
+        k_wgrad_few<<<dim3((nin + 255) / 256, (nout + kFewOut - 1) / kFewOut), 256, 0, st>>>(dz, ldz, x, ldx, rows,
+                                                                                             nout, nin, dw);
+        return cudaGetLastError();
+    }
     if (nin <= 16) return wgrad_shape<WgShape<16>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
     if (nin <= 256) return wgrad_shape<WgShape<144>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
     return wgrad_shape<WgShape<288>>(dz, ldz, x, ldx, rows, nout, nin, scratch, dw, st);
