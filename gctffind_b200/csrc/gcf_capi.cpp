@@ -1671,9 +1671,12 @@ bool rescale_lines_supported(int w, int h, int nw, int nh)
 // and a product's last wave is filled by the other lane's next one.  (64
 // micrographs of the uneven batch, 37 of them rescaled: 24.3 -> 20.3 ms a call.)
 // An image of the same size as its lane's last one finds the crop maps there.
+// Where the device has no memory for the second lane's scratch, all images take
+// the first lane.
 struct RescaleLanes {
     gcf_ctx* ctx;
     int used = 0;            // images placed
+    bool single = false;     // no memory for the second lane
     bool forked = false;
     struct Maps {
         int w = 0, h = 0, nw = 0, nh = 0;
@@ -1687,11 +1690,36 @@ struct RescaleLanes {
     // rescaled images and its scratch, which the next call's work on the
     // compute stream uses again.
     ~RescaleLanes() { join(); }
-    // The lane of the next image; the first use of the second lane orders it
-    // after everything on the compute stream.
-    gcf_status next(int* lane, cudaStream_t* st)
+    // Scratch of lane k for `bf` BF16 values and `f32` floats.
+    cudaError_t ensure(int k, size_t bf, size_t f32)
     {
+        cudaError_t e = ctx->rsg_bf[k].ensure(bf);
+        return e == cudaSuccess ? ctx->rsg_f[k].ensure(f32) : e;
+    }
+    // The same for the second lane: gives it up where there is no memory.
+    cudaError_t ensure_second(size_t bf, size_t f32)
+    {
+        if (ctx->capturing && (bf > ctx->rsg_bf[1].n || f32 > ctx->rsg_f[1].n)) {
+            single = true;   // nothing can be allocated now: the eager calls gave it up
+            return cudaSuccess;
+        }
+        const cudaError_t e = ensure(1, bf, f32);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        ctx->rsg_bf[1].release();
+        ctx->rsg_f[1].release();
+        single = true;
+        return cudaSuccess;
+    }
+    // The lane of the next image and its scratch; the first use of the second
+    // lane orders it after everything on the compute stream.
+    gcf_status next(const RescaleGemmLayout& L, int* lane, cudaStream_t* st)
+    {
+        const size_t bf = (size_t)L.bf16_elems, f32 = (size_t)L.f32_elems;
         *lane = used++ & 1;
+        if (*lane && !single) CK(ensure_second(bf, f32));
+        if (single) *lane = 0;
+        if (!*lane) CK(ensure(0, bf, f32));
         *st = *lane ? ctx->st_tile : ctx->st;
         if (*lane && !forked) {
             for (cudaEvent_t* e : {&ctx->rs_fork, &ctx->rs_join})
@@ -1717,10 +1745,9 @@ struct RescaleLanes {
             f32[u & 1] = std::max(f32[u & 1], (size_t)L.f32_elems);
             ++u;
         }
-        for (int k = 0; k < 2; ++k) {
-            if (bf[k]) CK(ctx->rsg_bf[k].ensure(bf[k]));
-            if (f32[k]) CK(ctx->rsg_f[k].ensure(f32[k]));
-        }
+        if (bf[0]) CK(ensure(0, bf[0], f32[0]));
+        if (bf[1]) CK(ensure_second(bf[1], f32[1]));
+        if (single) CK(ensure(0, std::max(bf[0], bf[1]), std::max(f32[0], f32[1])));
         return GCF_OK;
     }
     // The compute stream continues after both lanes.
@@ -1773,9 +1800,7 @@ gcf_status rescale_device(gcf_ctx* ctx, const float* img, int w, int h, float px
         const RescaleGemmLayout L = rescale_gemm_layout(w, h, nw, nh);
         int k = 0;
         cudaStream_t st = nullptr;
-        CKS(lanes.next(&k, &st));
-        CK(ctx->rsg_bf[k].ensure((size_t)L.bf16_elems));
-        CK(ctx->rsg_f[k].ensure((size_t)L.f32_elems));
+        CKS(lanes.next(L, &k, &st));
         RescaleLanes::Maps& mp = lanes.maps[k];
         const bool have = mp.w == w && mp.h == h && mp.nw == nw && mp.nh == nh && mp.at == ctx->rsg_bf[k].p;
         mp = {w, h, nw, nh, ctx->rsg_bf[k].p};

@@ -35,3 +35,25 @@ def test_failed_call_leaves_no_lane_running(gpu_lib, n):
             _batch(ctx, G, other + [small])
         assert _batch(ctx, G, good) == want
     ctx.close()
+
+
+def test_one_lane_where_memory_is_short(gpu_lib):
+    """With everything of a call allocated but the second lane's scratch, and
+    less device memory left than that takes, the call runs on one lane."""
+    import torch
+    G = gpu_lib
+    ctx = G.Context(0, 512, 0)
+    imgs = [img for seed in (100, 500) for img in _imgs(1, 5760, 4092, seed)]
+    ctx.set_rescale_impl(G.GCF_RESCALE_LINES)
+    _batch(ctx, G, imgs)                        # all but the lanes' scratch
+    ctx.set_rescale_impl(G.GCF_RESCALE_GEMM)
+    _batch(ctx, G, imgs[:1])                    # the first lane's (about 150 MB)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hold = torch.empty(free - (64 << 20), dtype=torch.uint8, device="cuda")
+    got = _batch(ctx, G, imgs)
+    del hold
+    torch.cuda.empty_cache()
+    assert _batch(ctx, G, imgs) == got          # on two lanes
+    ctx.close()
