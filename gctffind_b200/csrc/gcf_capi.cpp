@@ -806,7 +806,19 @@ gcf_status fused_plan(gcf_ctx* ctx, const std::vector<MicImage>& mics)
         tiles += nt;
         if (nch > 0) longest = std::max(longest, (nt + nch - 1) / nch);
     }
-    const bool single = tiles < 8 * longest;
+    // Each of them keeps a partial spectrum (526 KB, so at most 8 x 24 of them
+    // take 101 MB; an item takes one): where that is not to be had, whole items.
+    bool single = tiles < 8 * longest;
+    const size_t partials = (size_t)tiles * cx * T;
+    if (single && partials > ctx->f_partial.n) {
+        const cudaError_t e = ctx->capturing ? cudaErrorMemoryAllocation : ctx->f_partial.ensure(partials);
+        if (e == cudaErrorMemoryAllocation) {
+            if (!ctx->capturing) cudaGetLastError();
+            single = false;
+        } else {
+            CK(e);
+        }
+    }
     size_t nblk = 0;
     for (int i = 0; i < nm; ++i) {
         const MicImage& m = mics[i];

@@ -32,3 +32,31 @@ def test_items_in_a_row_keep_the_bits(gpu_lib, w, h):
     want = _raw(G, img, 816)[0]
     for got in _raw(G, img, 8):
         assert np.array_equal(got, want)
+
+
+def test_whole_items_where_memory_is_short(gpu_lib):
+    """A frame whose tiles are handed out singly keeps a partial spectrum per
+    tile (169 of them, 89 MB); with less device memory left it runs on whole
+    items, to the same bits."""
+    import torch
+    G = gpu_lib
+    g = torch.Generator(device="cuda").manual_seed(3)
+    img = torch.poisson(torch.full((3710, 3838), 5.0, device="cuda"), generator=g)
+    other = img[:1024, :1024].contiguous()
+    ctx = G.Context(0, 512, 0)
+
+    def raw(x):
+        ctx.setup(G.make_optics(pixel_size=1.3), x.shape[1], x.shape[0])
+        ctx.gen_half_spectrum(x)
+        return ctx.half_spectrum(raw=True)
+
+    raw(other)                                  # all buffers but the larger frame's partials
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hold = torch.empty(free - (48 << 20), dtype=torch.uint8, device="cuda")
+    short = raw(img)
+    del hold
+    torch.cuda.empty_cache()
+    assert np.array_equal(raw(img), short)      # singly
+    ctx.close()
