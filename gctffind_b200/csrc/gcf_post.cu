@@ -551,7 +551,10 @@ cudaError_t launch_background(const float* raw, int tile, int nmic, int log_spec
     const BgShape b = bg_shape(tile, nmic);
     const int ew = (b.strip + 2 * (b.box / 2) + 31) & ~31;
     const int threads = ew * std::max(1, (b.smem > kTwoPerSM ? 1024 : kBgThreads) / ew);
-    cudaError_t e = cudaFuncSetAttribute(k_background, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
+    // the same limit on every call: the attribute is the process's, and another
+    // thread's context may have a tile that needs less
+    if (b.smem > kOnePerSM) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaFuncSetAttribute(k_background, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOnePerSM);
     if (e != cudaSuccess) return e;
     k_background<<<dim3(b.blocks(tile), nmic), threads, b.smem, st>>>(raw, tile, log_spect, b.box, b.seg, b.strip,
                                                                          ctf, part, ticket, mom);
