@@ -1256,7 +1256,9 @@ gcf_status run_search_enqueue(gcf_ctx* ctx, const std::vector<JobSpec>& specs, S
 gcf_status check_dev_err(gcf_ctx* ctx, int flag)
 {
     if (!flag) return GCF_OK;
-    CK(cudaMemset(ctx->dev_err.p, 0, sizeof(int)));
+    // on the stream that every call starts from: the next call's spectra (void
+    // where the flag is set, see k_item_reduce) come after it
+    CK(cudaMemsetAsync(ctx->dev_err.p, 0, sizeof(int), ctx->st));
     return fail(ctx, GCF_ERR_TIMEOUT, "tile spectrum or tensor-core rescale: a bounded wait gave up");
 }
 
