@@ -51,13 +51,13 @@ sys.path.insert(0, ROOT)
 N_BATCH = 256
 METRIC = "4096^2 micrographs/s, learned+batched+BF16 vs plain GPU path; defocus error (A)"
 SERIES_PX = 1.35
-# DRAM bytes (read + write) of k_fused_spectrum per algorithmic byte (the
+# DRAM bytes (read + write) of k_fused_spectrum_pair per algorithmic byte (the
 # images read once), from ncu dram__bytes_read.sum + dram__bytes_write.sum of
 # the first tile launch of `bench.py --batch 16 --steps 1 --warmup 3
 # --no-secondary --no-cpu-baseline --no-autotune --no-graphs --mode bf16`
 # (16 micrographs of this workload, 904.6 MB of algorithmic bytes)
-TILE_KERNEL_TRAFFIC_RATIO = (1_028_731_000 + 62_378_752) / 904_559_168
-TILE_KERNEL_TRAFFIC_CAPTURE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the first k_fused_spectrum launch "
+TILE_KERNEL_TRAFFIC_RATIO = (1_973_598_720 + 39_013_632) / 904_559_168
+TILE_KERNEL_TRAFFIC_CAPTURE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the first k_fused_spectrum_pair launch "
                                "of bench.py --batch 16 (16 micrographs of this workload), per algorithmic byte, "
                                "scaled by this launch's algorithmic bytes")
 
@@ -468,7 +468,7 @@ def h2d_rate(src, device):
 
 
 def tile_kernel_roofline(stage, imgs_dims, pk):
-    """k_fused_spectrum (+ its cluster-less companion) over every tile of the
+    """k_fused_spectrum_pair (+ its cluster-less companion) over every tile of the
     batch: algorithmic bytes = each (rescaled) image the kernel reads, read
     once; time = the union of its launches inside the timed calls."""
     ms = stage.get("tile_kernel", 0.0)
@@ -481,7 +481,7 @@ def tile_kernel_roofline(stage, imgs_dims, pk):
     tiles = sum(max(0, (w - 256) // 256) * max(0, (h - 256) // 256) for w, h in imgs_dims)
     flops = tiles * (2.5 * 512 * 512 * 18 + 6 * 512 * 512)
     tflops = flops / (ms / 1000.0) / 1e12 if ms > 0 else 0.0
-    return {"kernel": "k_fused_spectrum (8-CTA clusters) + k_fused_spectrum_solo (the SMs the clusters leave free)",
+    return {"kernel": "k_fused_spectrum_pair (8-CTA clusters) + k_fused_spectrum_solo (the SMs the clusters leave free)",
             "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "peak_source": "fallback" if pk.get("_fallback") else "measured",
             "traffic": int(algo * TILE_KERNEL_TRAFFIC_RATIO),
