@@ -451,7 +451,7 @@ void launch_concat(const __nv_bfloat16* x1, const __nv_bfloat16* y4, int B, __nv
 // zero); scratch: kWgSlices x (the largest tile's and bias's floats), see
 // wgrad_scratch_floats
 constexpr int kWgSlices = 148;
-constexpr size_t wgrad_scratch_floats() { return (size_t)kWgSlices * 32 * (288 + 1) + 256 * (2304 + 1) * 2; }
+constexpr size_t wgrad_scratch_floats() { return (size_t)kWgSlices * 32 * (288 + 2) + 256 * (2304 + 2) * 2; }
 cudaError_t launch_wgrad(const __nv_bfloat16* dz, long long ldz, const __nv_bfloat16* x, long long ldx, int rows,
                          int nout, int nin, float* scratch, float* dw, cudaStream_t st);
 void launch_mse(const float* pred, long long ldp, const float* target, int B, float* loss, __nv_bfloat16* dpred,

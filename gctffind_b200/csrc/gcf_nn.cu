@@ -469,9 +469,12 @@ __global__ void k_concat(const __nv_bfloat16* __restrict__ x1, const __nv_bfloat
 // a ring of kWgStages shared-memory stages (cp.async, 16 bytes).  Its eight
 // warps split the KT columns into groups of CW and the rows of a chunk among
 // the warps of a group.  Products are exact in FP32; a warp's tensor-core sums
-// are added to FP32 registers every kWgFlush chunks, so that no long chain
-// keeps the tensor core's truncation.
-constexpr int kWgStages = 4, kWgFlush = 4;
+// are added to FP32 registers after every chunk, so that no long chain keeps the
+// tensor core's truncation.  (Every four chunks it showed where a slice has
+// several: 256 x 2304 outputs of 512 rows, two slices, 1.37e-7, against 7.1e-8
+// now and the scalar kernel's 1.11e-7; the times are the same, 13.1 us at 256
+// rows and 50.2 at 4096.)  The biases are FP64 sums of eight rows each.
+constexpr int kWgStages = 4;
 
 template <int KT_>
 struct WgShape {
@@ -500,10 +503,10 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok)
 template <class S>
 __global__ void __launch_bounds__(256, 1)
 k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16* __restrict__ x, long long ldx,
-        int rows, int nout, int nin, int rows_per_cta, float* __restrict__ part, float* __restrict__ part_b)
+        int rows, int nout, int nin, int rows_per_cta, float* __restrict__ part, double* __restrict__ part_b)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
-    __shared__ float sb[8][32];
+    __shared__ double sb[8][32];
     const int k0 = blockIdx.x * S::KT, o0 = blockIdx.y * 32;
     const int r0 = blockIdx.z * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -528,7 +531,8 @@ k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[2][S::NT][4], sum[2][S::NT][4], bsum = 0.0f;
+    float acc[2][S::NT][4], sum[2][S::NT][4];
+    double bsum = 0.0;
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -542,7 +546,13 @@ k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16
         fill(c + kWgStages - 1);
         const __nv_bfloat16 *X = xs(c % kWgStages), *Z = zs(c % kWgStages);
         if (blockIdx.x == 0)   // bias: this thread's column and eighth of the rows
-            for (int r = warp; r < S::ROWS; r += 8) bsum += bf(Z[r * S::ZP + lane]);
+#pragma unroll
+            for (int r = warp; r < S::ROWS; r += 64) {
+                float b = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) b += bf(Z[(r + 8 * i) * S::ZP + lane]);
+                bsum += (double)b;
+            }
 #pragma unroll
         for (int t = 0; t < S::STEPS; ++t) {
             const int rr = (rg * S::STEPS + t) * 16;
@@ -574,17 +584,15 @@ k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16
                         : "r"(af[m][0]), "r"(af[m][1]), "r"(af[m][2]), "r"(af[m][3]), "r"(b0), "r"(b1));
             }
         }
-        if ((c + 1) % kWgFlush == 0 || c + 1 == nch) {
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-                for (int n = 0; n < S::NT; ++n)
+            for (int n = 0; n < S::NT; ++n)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        sum[m][n][i] += acc[m][n][i];
-                        acc[m][n][i] = 0.0f;
-                    }
-        }
+                for (int i = 0; i < 4; ++i) {
+                    sum[m][n][i] += acc[m][n][i];
+                    acc[m][n][i] = 0.0f;
+                }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();   // the ring is free: the warps' sums, [row group][output][column]
@@ -610,7 +618,7 @@ k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16
         part[((size_t)blockIdx.z * nout + o) * nin + k] = v;
     }
     if (blockIdx.x == 0 && tid < 32 && o0 + tid < nout) {
-        float v = 0.0f;
+        double v = 0.0;
         for (int w = 0; w < 8; ++w) v += sb[w][tid];
         part_b[(size_t)blockIdx.z * nout + o0 + tid] = v;
     }
@@ -618,16 +626,20 @@ k_wgrad(const __nv_bfloat16* __restrict__ dz, long long ldz, const __nv_bfloat16
 
 // dw[i] = sum of the slices' part[z][i], i < n (the bias after the weights),
 // in FP64 in slice order
-__global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ part, const float* __restrict__ part_b,
-                                                   int slices, int nw, int nb, float* __restrict__ dw)
+__global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ part,
+                                                   const double* __restrict__ part_b, int slices, int nw, int nb,
+                                                   float* __restrict__ dw)
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= nw + nb) return;
-    const float* p = i < nw ? part + i : part_b + (i - nw);
-    const size_t st = i < nw ? nw : nb;
     double s = 0.0;
+    if (i < nw) {
 #pragma unroll 8
-    for (int z = 0; z < slices; ++z) s += (double)__ldg(p + z * st);
+        for (int z = 0; z < slices; ++z) s += (double)__ldg(part + i + (size_t)z * nw);
+    } else {
+#pragma unroll 8
+        for (int z = 0; z < slices; ++z) s += __ldg(part_b + (i - nw) + (size_t)z * nb);
+    }
     dw[i] = (float)s;
 }
 
@@ -813,7 +825,7 @@ static cudaError_t wgrad_shape(const __nv_bfloat16* dz, long long ldz, const __n
     slices = (rows + per - 1) / per;
     cudaError_t e = cudaFuncSetAttribute(k_wgrad<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
     if (e != cudaSuccess) return e;
-    float* part_b = scratch + (size_t)slices * nout * nin;
+    double* part_b = reinterpret_cast<double*>(scratch + (size_t)slices * nout * nin);   // nin is even
     k_wgrad<S><<<dim3(gx, gy, slices), 256, S::SMEM, st>>>(dz, ldz, x, ldx, rows, nout, nin, per, scratch, part_b);
     const int nw = nout * nin;
     k_wgrad_sum<<<(nw + nout + 255) / 256, 256, 0, st>>>(scratch, part_b, slices, nw, nout, dw);
